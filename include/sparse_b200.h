@@ -401,8 +401,10 @@ int sb_spts_plan_reordered(const sb_spts_plan* plan, int32_t* row_ptr, int32_t* 
  * src/parallel/src/spts_opt_32.wat:339-546), SB_SPTS_SYNCFREE replaces
  * spts_csr_sync_free (src/parallel/src/spts_opt_32.wat:8-260) and
  * SB_SPTS_HYBRID replaces spts_csr_opt_level_sync_free
- * (src/parallel/src/sparse_opt_32.wat:12846-13445).  Stream-ordered; a
- * dependency wait that runs out is reported by sb_device_status (code 2). */
+ * (src/parallel/src/sparse_opt_32.wat:12846-13445).  LEVEL and HYBRID have
+ * the same arithmetic, so the kernel follows the factor's shape, not the name.
+ * Stream-ordered; a dependency wait that runs out is reported by
+ * sb_device_status (code 2). */
 int sb_spts_solve(const sb_spts_plan* plan, int algo, int policy, const void* b, void* y,
                   void* stream);
 
@@ -453,7 +455,8 @@ int sb_spts_plan_growth(const sb_spts_plan* plan, double* growth, void* stream);
 
 /* Batched solves (no counterpart in the reference, which solves one system
  * per call): many independent systems, each with its own analysed plan, in
- * one persistent launch replayed from a captured CUDA graph.  Every row is
+ * one CUDA graph (factors with a window layout one per block, the others in
+ * one launch with ready flags).  Every row is
  * solved with the arithmetic of SB_SPTS_HYBRID, so each result is
  * bit-identical to sb_spts_solve(plan, SB_SPTS_HYBRID, policy, b, y).  An
  * executor serves one value dtype (SB_F32 or SB_F64) and one accumulation
@@ -477,8 +480,9 @@ int sb_spts_batch_create(int dtype, int policy, int32_t capacity, sb_spts_batch*
 int sb_spts_batch_destroy(sb_spts_batch* e);
 int sb_spts_batch_run(sb_spts_batch* e, const sb_spts_batch_item* items, int32_t n,
                       void* stream);
-/* Launch shape of later runs: blocks_per_sm 0 (the default) launches one warp
- * per 32-row chunk, resident blocks capped by the batch size; > 0 launches at
+/* Launch shape of later runs (of the solves with ready flags; those with one
+ * factor per block keep to the same cap): blocks_per_sm 0 (the default)
+ * launches one warp per 32-row chunk, resident blocks capped by the batch size; > 0 launches at
  * most that many blocks per SM (and no more than fit), whose warps take
  * chunks until the batch is done, so that a run leaves SMs to work on other
  * streams (for instance a second executor's run). */

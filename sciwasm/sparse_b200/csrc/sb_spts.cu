@@ -16,15 +16,19 @@
 // the results are bit-identical to the reference's row kernels):
 //   SB_SPTS_LEVEL    level by level on the reordered matrix, the row kernel
 //                    of src/parallel/src/sparse_opt_32.wat:11679-11757
-//                    (t = 0; t += L_ij*y_j; y_i = (b_i - t)/L_ii), in one
-//                    cooperative launch with a grid barrier per level
+//                    (t = 0; t += L_ij*y_j; y_i = (b_i - t)/L_ii)
 //   SB_SPTS_SYNCFREE natural order with per-row ready flags, the kernel of
 //                    src/parallel/src/spts_opt_32.wat:8-117
 //                    (t = b_i; t -= L_ij*y_j; y_i = t/L_ii)
 //   SB_SPTS_HYBRID   level order with ready flags (no per-level barrier), the
 //                    row kernel's arithmetic, as the level/sync-free hybrid of
 //                    src/parallel/src/sparse_opt_32.wat:12846-13445
+// SB_SPTS_LEVEL and SB_SPTS_HYBRID have the same arithmetic, so the kernel is
+// chosen by the factor's shape (solve_impl): one block with its values in
+// shared memory (sb_spts_window.cuh), one block with a barrier per level, or
+// ready flags over the whole GPU.
 #include <algorithm>
+#include <climits>
 #include <cstring>
 #include <type_traits>
 #include <mutex>
@@ -32,6 +36,7 @@
 
 #include "sb_common.cuh"
 #include "sb_prims.cuh"
+#include "sb_spts_window.cuh"
 
 struct sb_spts_plan {
   int dtype = 0;
@@ -52,7 +57,11 @@ struct sb_spts_plan {
   void* rval = nullptr;
   void* ywork = nullptr;
   int* ticket = nullptr;
-  std::vector<int> h_level_ptr;
+  // window layout (in the memory of rcol and rval, which are then not stored)
+  sb::win::Info window = {};
+  int ngroups = 0;
+  int4* groups = nullptr;
+  char* records = nullptr;
   std::vector<void*> owned;
   cudaEvent_t ev[2] = {nullptr, nullptr};  // bracket the analysis's device work
   float analysis_ms = 0.f;
@@ -115,19 +124,6 @@ __device__ __forceinline__ int next_rows(int* ticket) {
   if ((threadIdx.x & 31) == 0) base = atomicAdd(ticket, 32);
   return __shfl_sync(0xffffffffu, base, 0);
 }
-
-template <typename T> __device__ __forceinline__ T mul_rn(T a, T b);
-template <> __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-template <> __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-template <typename T> __device__ __forceinline__ T add_rn(T a, T b);
-template <> __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
-template <> __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
-template <typename T> __device__ __forceinline__ T sub_rn(T a, T b);
-template <> __device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
-template <> __device__ __forceinline__ double sub_rn(double a, double b) { return __dsub_rn(a, b); }
-template <typename T> __device__ __forceinline__ T div_rn(T a, T b);
-template <> __device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, b); }
-template <> __device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(a, b); }
 
 // ------------------------------------------------------------ pending values
 // The plan-based solves and the level analysis publish each row's result in a
@@ -317,19 +313,15 @@ __global__ void perm_order(const unsigned* __restrict__ sorted_rows, int N, int*
   }
 }
 
-__global__ void gather_lengths(const int* __restrict__ row_ptr, const int* __restrict__ perm,
-                               int N, int* __restrict__ lens) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < N) lens[p] = row_ptr[perm[p] + 1] - row_ptr[perm[p]];
-}
-
+// Not run where the window layout takes the memory (info->use).
 template <typename T>
 __global__ void reorder_rows(const int* __restrict__ row_ptr, const int* __restrict__ col,
                              const T* __restrict__ val, const int* __restrict__ perm,
                              const int* __restrict__ order, const int* __restrict__ rrow, int N,
-                             int* __restrict__ rcol, T* __restrict__ rval) {
+                             const win::Info* __restrict__ info, int* __restrict__ rcol,
+                             T* __restrict__ rval) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= N) return;
+  if (p >= N || info->use) return;
   const int src = perm[p];
   int o = rrow[p];
   for (int j = row_ptr[src]; j < row_ptr[src + 1]; ++j, ++o) {
@@ -340,74 +332,6 @@ __global__ void reorder_rows(const int* __restrict__ row_ptr, const int* __restr
 }
 
 // ------------------------------------------------------------ solves
-
-// Row kernel of the level-set solve on rows [r0, r1) of the reordered matrix;
-// b is read through the permutation, y is kept in level order.
-template <typename T, typename A>
-__global__ void spts_level_rows(const int* __restrict__ rrow, const int* __restrict__ rcol,
-                                const T* __restrict__ rval, int r0, int r1,
-                                const int* __restrict__ perm, const T* __restrict__ b,
-                                T* __restrict__ yw) {
-  const int i = r0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= r1) return;
-  const int s = rrow[i], end = rrow[i + 1] - 1;
-  const A bi = (A)b[perm[i]];
-  if (end > s) {
-    A t = 0;
-    for (int j = s; j < end; ++j) t = add_rn(t, mul_rn((A)rval[j], (A)yw[rcol[j]]));
-    yw[i] = (T)div_rn(sub_rn(bi, t), (A)rval[end]);
-  } else {
-    yw[i] = (T)div_rn(bi, (A)rval[end]);
-  }
-}
-
-// Grid barrier of a cooperative launch (every block resident) on one
-// monotonic arrival counter: at the barrier that closes level l, thread 0 of
-// each block adds 1 with an acquire-release add (ordered after the block's
-// stores, which bar.sync made visible to it) and waits until the counter reaches
-// gridDim.x * (l + 1), polling with acquire loads and a short sleep, bounded
-// by `limit` SM cycles (or by a timeout already recorded in the status
-// word).  One atomic per block and level: no reset and no generation word
-// (the earlier form's last arrival reset the counter and advanced a
-// generation, two more dependent atomics per level).  The comparison is
-// wrap-safe: the counter never runs more than gridDim.x ahead of a waiter.
-// Returns false after a timeout, which it records; the caller then returns.
-__device__ __forceinline__ unsigned atom_add_acq_rel(unsigned* p, unsigned v) {
-  unsigned old;
-  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;"
-               : "=r"(old) : "l"(p), "r"(v) : "memory");
-  return old;
-}
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, long long limit,
-                                             int* status) {
-  __shared__ int ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ok = 1;
-    // acq_rel: the last block to arrive goes on at once, so its add also
-    // acquires the other blocks' released stores
-    if (atom_add_acq_rel(bar, 1u) + 1u != target) {
-      const long long t0 = clock64();
-      unsigned ns = SB_SPTS_SLEEP_MIN_NS;
-      while ((int)(ld_acquire_u32(bar) - target) < 0) {
-        if (clock64() - t0 > limit || *(volatile const int*)status) {
-          atomicExch(status, SB_DEV_TIMEOUT_DEP);
-          ok = 0;
-          break;
-        }
-        __nanosleep(ns);
-        ns = ns < SB_SPTS_SLEEP_MAX_NS ? 2 * ns : ns;
-      }
-    }
-  }
-  __syncthreads();
-  return ok != 0;
-}
 
 // A thread's first row of a level, read ahead of the barrier that opens the
 // level: its structure, b, diagonal and up to kG off-diagonal columns and
@@ -473,31 +397,28 @@ __device__ __forceinline__ void level_row_load(LevelRow<T, A>& r, int i, const i
   }
 }
 
-// The level-set solve in one cooperative launch: the levels in order, the
-// rows of a level spread over all threads with the arithmetic of
-// spts_level_rows, a grid barrier after every level (the reference's
-// structure, src/parallel/src/spts_opt_32.wat:339-546).  Values of earlier
-// levels are read from L2 (__ldcg), since L1 is not kept coherent with other
-// SMs' stores inside a launch; each row also writes its natural-order
-// output, so no scatter pass follows.  Each thread reads its first row of
-// a level in two rounds ahead of time: its row pointers and permutation two
-// levels before, its columns, values, b and diagonal one level before, so
-// that only the y reads after each barrier lie on the level's critical
-// path.  When every level fits in
-// one block of kLevelBlock1 threads, the launch is that one block and the
-// barrier is __syncthreads.
-constexpr int kLevelBlock1 = 512;  // threads of the single-block form
+// The level-set solve of a factor whose levels all fit one block of
+// kLevelBlock threads: the levels in order, one row per thread, a block barrier
+// after every level (the reference's structure,
+// src/parallel/src/spts_opt_32.wat:339-546).  Values of earlier levels are
+// read from L2 (__ldcg); each row also writes its natural-order output, so no
+// scatter pass follows.  Each thread reads its row of a level ahead of time
+// (TWO: in two rounds, its row pointers and permutation two levels before, its
+// columns, values, b and diagonal one level before), so that only the y reads
+// after each barrier lie on the level's critical path.  Wider levels go to the
+// ready flags of spts_hybrid_rows: a grid barrier per level measured 2.1 us
+// per level against their 1.3 (3-D Laplacian 64^3 FP64, 0.41 and 0.25 ms).
+constexpr int kLevelBlock = 512;
 
 template <typename T, typename A, bool TWO>
-__global__ void __launch_bounds__(kLevelBlock1, 1)
-    spts_level_coop(const int* __restrict__ rrow, const int* __restrict__ rcol,
-                    const T* __restrict__ rval, const int* __restrict__ level_ptr, int nlevels,
-                    const int* __restrict__ perm, const T* __restrict__ b, T* yw,
-                    T* __restrict__ y, unsigned* bar, long long limit, int* status) {
-  const int nthreads = gridDim.x * blockDim.x;
-  const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kLevelBlock, 1)
+    spts_level_block(const int* __restrict__ rrow, const int* __restrict__ rcol,
+                     const T* __restrict__ rval, const int* __restrict__ level_ptr, int nlevels,
+                     const int* __restrict__ perm, const T* __restrict__ b, T* yw,
+                     T* __restrict__ y) {
+  const int gt = threadIdx.x;
   LevelRow<T, A> nx;
-  LevelHead hd;  // the first row of the level after the next one
+  LevelHead hd;  // the row of the level after the next one
   {
     const int r0 = __ldg(level_ptr), r1 = __ldg(level_ptr + 1);
     if (r0 + gt < r1) level_row_load(nx, r0 + gt, rrow, rcol, rval, perm, b);
@@ -507,8 +428,8 @@ __global__ void __launch_bounds__(kLevelBlock1, 1)
     }
   }
   for (int l = 0; l < nlevels; ++l) {
-    const int r0 = __ldg(level_ptr + l), r1 = __ldg(level_ptr + l + 1);
-    if (nx.i >= 0) {  // the prefetched first row (index r0 + gt)
+    const int r1 = __ldg(level_ptr + l + 1);
+    if (nx.i >= 0) {
       A t = 0;
       const int n = nx.end - nx.s;
       T w[kG];
@@ -524,26 +445,11 @@ __global__ void __launch_bounds__(kLevelBlock1, 1)
       __stcg(yw + nx.i, yi);
       y[nx.pi] = yi;
     }
-    for (int i = r0 + gt + nthreads; i < r1; i += nthreads) {
-      const int s = rrow[i], end = rrow[i + 1] - 1;
-      const int pi = perm[i];
-      const A bi = (A)b[pi];
-      T yi;
-      if (end > s) {
-        A t = 0;
-        for (int j = s; j < end; ++j) t = add_rn(t, mul_rn((A)rval[j], (A)__ldcg(yw + rcol[j])));
-        yi = (T)div_rn(sub_rn(bi, t), (A)rval[end]);
-      } else {
-        yi = (T)div_rn(bi, (A)rval[end]);
-      }
-      __stcg(yw + i, yi);
-      y[pi] = yi;
-    }
     if (l + 1 < nlevels) {
       if constexpr (TWO) {
-        // the next level's first row from the head read one level ago, and
-        // the head of the level after it: neither depends on y, so both load
-        // rounds overlap the barrier and the next level's y reads
+        // the next level's row from the head read one level ago, and the head
+        // of the level after it: neither depends on y, so both load rounds
+        // overlap the barrier and the next level's y reads
         level_row_from_head(nx, hd, rcol, rval, b);
         hd.i = -1;
         if (l + 2 < nlevels) {
@@ -551,13 +457,12 @@ __global__ void __launch_bounds__(kLevelBlock1, 1)
           if (q0 + gt < q1) level_head_load(hd, q0 + gt, rrow, perm);
         }
       } else {
-        // both rounds of the next level's first row, before the barrier
-        const int q0 = r1, q1 = __ldg(level_ptr + l + 2);
+        // both rounds of the next level's row, before the barrier
+        const int q1 = __ldg(level_ptr + l + 2);
         nx.i = -1;
-        if (q0 + gt < q1) level_row_load(nx, q0 + gt, rrow, rcol, rval, perm, b);
+        if (r1 + gt < q1) level_row_load(nx, r1 + gt, rrow, rcol, rval, perm, b);
       }
-      if (gridDim.x == 1) __syncthreads();  // one block: its barrier orders the L2 accesses
-      else if (!grid_barrier(bar, gridDim.x * (unsigned)(l + 1), limit, status)) return;
+      __syncthreads();  // orders the block's L2 accesses
     }
   }
 }
@@ -665,15 +570,10 @@ __global__ void spts_syncfree_rows(const int* __restrict__ row_ptr, const int* _
   }
 }
 
-template <typename T>
-__global__ void scatter_by_perm(const T* __restrict__ yw, const int* __restrict__ perm, int N,
-                                T* __restrict__ y) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < N) y[perm[p]] = yw[p];
-}
-
 // ------------------------------------------------------------ batched solves
-// Many independent systems in one launch of one warp per 32-row chunk (not
+// Plans with a window layout are solved one per block
+// (win::window_solve_many); the others as follows.  Many independent systems
+// in one launch of one warp per 32-row chunk (not
 // persistent: warps exit after their chunk, and the hardware dispatches the
 // blocks as SM slots free up).  Warps are laid out in rounds of one chunk per
 // unfinished system, so all systems of a batch advance at the same time and
@@ -950,18 +850,59 @@ static int analyze_impl(sb_spts_plan* p, cudaStream_t st) {
   level_hist<<<grid1(N), kT, 0, st>>>(p->level, N, p->level_ptr);
   SB_CHECK_LAUNCH("level_hist");
   if ((r = prim::exclusive_scan(p->level_ptr, p->level_ptr, L + 1, st))) return r;
-  // stable counting sort of rows by level
+  // stable counting sort of rows by level; scratch: sort buffers, then the
+  // window layout's counts
+  const int gmax = N / win::kGroup + L + 1;  // no more groups than this
   prim::RadixBuffers rb;
   void* mem = nullptr;
-  const size_t kb = sizeof(unsigned long long) * N, vb = sizeof(unsigned) * N;
-  if ((r = scratch_alloc(&mem, 2 * kb + 2 * vb, st))) return r;
-  rb.k[0] = (unsigned long long*)mem;
-  rb.k[1] = (unsigned long long*)((char*)mem + kb);
-  rb.v[0] = (unsigned*)((char*)mem + 2 * kb);
-  rb.v[1] = (unsigned*)((char*)mem + 2 * kb + vb);
-  level_keys<<<grid1(N), kT, 0, st>>>(p->level, N, rb.k[0], rb.v[0]);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) r = cuda_status(e, "level_keys");
+  const size_t kb = align256(sizeof(unsigned long long) * N), vb = align256(sizeof(unsigned) * N);
+  const size_t gb = align256(sizeof(int) * ((size_t)gmax + 1));
+  const size_t lb = align256(sizeof(int) * ((size_t)L + 1));
+  if ((r = scratch_alloc(&mem, 2 * kb + 2 * vb + lb + 2 * gb + 256, st))) return r;
+  char* q = (char*)mem;
+  rb.k[0] = (unsigned long long*)q;
+  rb.k[1] = (unsigned long long*)(q + kb);
+  rb.v[0] = (unsigned*)(q + 2 * kb);
+  rb.v[1] = (unsigned*)(q + 2 * kb + vb);
+  q += 2 * kb + 2 * vb;
+  int* gstart = (int*)q;               // [L + 1] groups of the levels before
+  int* glen = (int*)(q + lb);          // [gmax + 1] longest row of a group
+  int* gbase = (int*)(q + lb + gb);    // [gmax + 1] first entry of a group
+  win::Info* info = (win::Info*)(q + lb + 2 * gb);
+  // where the window layout goes: the records in the memory of rcol and rval,
+  // the group descriptors behind level_ptr's L + 1 entries if they fit there,
+  // else at the end of rcol and rval
+  long long cap = -1;  // 16-byte units for the records
+  {
+    const size_t area = align256(sizeof(int) * (size_t)nnz) + align256(sizeof(T) * (size_t)nnz);
+    const size_t lp = align256(sizeof(int) * ((size_t)L + 1));
+    const size_t slack = align256(sizeof(int) * ((size_t)N + 2)) - lp;
+    const size_t gbytes = align256(sizeof(int4) * (size_t)gmax);
+    size_t room = area;
+    p->records = (char*)p->rcol;
+    if (gbytes <= slack) {
+      p->groups = (int4*)((char*)p->level_ptr + lp);
+    } else if (gbytes < area) {
+      room -= gbytes;
+      p->groups = (int4*)(p->records + room);
+    }
+    if (p->groups) cap = std::min<long long>((long long)(room / 16), INT_MAX / 2);
+  }
+  int4* groups = cap >= 0 ? p->groups : nullptr;
+  cudaError_t e = cudaMemsetAsync(gstart, 0, lb + 2 * gb + 256, st);
+  if (e != cudaSuccess) r = cuda_status(e, "sb_spts_analyze");
+  if (!r) {
+    win::window_reach<<<grid1(N), kT, 0, st>>>(p->row_ptr, p->col, p->level, p->level_ptr, N, info);
+    win::window_level_groups<<<grid1(L + 1), kT, 0, st>>>(p->level_ptr, L, gstart, info);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) r = cuda_status(e, "window_reach");
+    if (!r) r = prim::exclusive_scan(gstart, gstart, L + 1, st);
+  }
+  if (!r) {
+    level_keys<<<grid1(N), kT, 0, st>>>(p->level, N, rb.k[0], rb.v[0]);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) r = cuda_status(e, "level_keys");
+  }
   const int ranges[2] = {0, prim::bits_for(L - 1)};
   int which = 0;
   if (!r) r = prim::radix_sort_ranges(rb, N, ranges, 1, &which, st);
@@ -971,36 +912,87 @@ static int analyze_impl(sb_spts_plan* p, cudaStream_t st) {
     if (e != cudaSuccess) r = cuda_status(e, "perm_order");
   }
   if (!r) {
-    // reordered CSR: row lengths in level order, scanned into rrow
+    // row lengths in level order, scanned into rrow
     int* lens = (int*)rb.k[0];
-    gather_lengths<<<grid1(N), kT, 0, st>>>(p->row_ptr, p->perm, N, lens);
+    win::window_lengths<<<grid1(N), kT, 0, st>>>(p->row_ptr, p->perm, p->level, p->level_ptr,
+                                                 gstart, N, lens, groups, glen);
     e = cudaGetLastError();
-    if (e != cudaSuccess) r = cuda_status(e, "gather_lengths");
+    if (e != cudaSuccess) r = cuda_status(e, "window_lengths");
     if (!r) r = prim::exclusive_scan(lens, p->rrow, N, st);
     if (!r) {
       const int nz = (int)nnz;
       e = cudaMemcpyAsync(p->rrow + N, &nz, sizeof(int), cudaMemcpyHostToDevice, st);
       if (e != cudaSuccess) r = cuda_status(e, "rrow");
     }
+    if (!r && groups) {
+      win::window_sizes<<<grid1(gmax + 1), kT, 0, st>>>(groups, glen, gmax, gstart + L,
+                                                        sizeof(T), gbase, info);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) r = cuda_status(e, "window_sizes");
+      if (!r) r = prim::exclusive_scan(gbase, gbase, gmax + 1, st);
+      if (!r) {
+        win::window_decide<<<1, 1, 0, st>>>(gbase + gmax, gstart + L, L, cap, sizeof(T),
+                                             h[0] == 0, info);
+        win::window_fill<T><<<grid1(N), kT, 0, st>>>(
+            p->row_ptr, p->col, (const T*)p->val, p->perm, p->order, p->level, p->level_ptr, gstart,
+            glen, gbase, N, info, groups, p->records);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) r = cuda_status(e, "window_fill");
+      }
+    }
     if (!r) {
       reorder_rows<T><<<grid1(N), kT, 0, st>>>(p->row_ptr, p->col, (const T*)p->val, p->perm,
-                                                p->order, p->rrow, N, p->rcol, (T*)p->rval);
+                                                p->order, p->rrow, N, info, p->rcol, (T*)p->rval);
       e = cudaGetLastError();
       if (e != cudaSuccess) r = cuda_status(e, "reorder_rows");
     }
   }
   if (!r) {
-    p->h_level_ptr.resize((size_t)L + 1);
     e = cudaEventRecord(p->ev[1], st);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync(p->h_level_ptr.data(), p->level_ptr, sizeof(int) * ((size_t)L + 1),
-                          cudaMemcpyDeviceToHost, st);
+      e = cudaMemcpyAsync(&p->window, info, sizeof(win::Info), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(&p->ngroups, gstart + L, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = cudaEventElapsedTime(&p->analysis_ms, p->ev[0], p->ev[1]);
     if (e != cudaSuccess) r = cuda_status(e, "sb_spts_analyze");
   }
   scratch_free(mem, st);
   return r;
+}
+
+template <typename T>
+static win::View<T> window_view(const sb_spts_plan* p, T* yw) {
+  return {p->groups,         p->records,     yw, p->ngroups, p->window.window,
+          p->window.kmax, p->window.widest};
+}
+
+template <typename T, typename A, int KU>
+static int launch_window(const sb_spts_plan* p, T* yw, int* status, cudaStream_t st) {
+  auto k = win::window_solve<T, A, KU>;
+  SB_CHECK_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     win::kSmem));
+  k<<<1, 32 * win::Warps<T, KU>::n, win::smem_bytes(p->window.window, sizeof(T)), st>>>(
+      window_view(p, yw), status);
+  SB_CHECK_LAUNCH("window_solve");
+  return SB_OK;
+}
+
+// b into level order, the solve on one block, y back into natural order.
+template <typename T, typename A>
+static int solve_window(const sb_spts_plan* p, const T* b, T* y, int* status, cudaStream_t st) {
+  const int N = p->N;
+  T* yw = (T*)p->ywork;
+  win::gather_by_perm<T><<<grid1(N), kT, 0, st>>>(b, p->perm, N, yw);
+  SB_CHECK_LAUNCH("gather_by_perm");
+  const int u = win::unroll_of(p->window.kmax);
+  const int r = u == 4   ? launch_window<T, A, 4>(p, yw, status, st)
+                : u == 8 ? launch_window<T, A, 8>(p, yw, status, st)
+                         : launch_window<T, A, 16>(p, yw, status, st);
+  if (r) return r;
+  win::scatter_by_perm<T><<<grid1(N), kT, 0, st>>>(yw, p->perm, N, y);
+  SB_CHECK_LAUNCH("scatter_by_perm");
+  return SB_OK;
 }
 
 template <typename T, typename A>
@@ -1012,71 +1004,32 @@ static int solve_impl(const sb_spts_plan* p, int algo, const T* b, T* y, long lo
     set_error("sb_spts_solve: device status word unavailable");
     return SB_ENOMEM;
   }
+  if (algo != SB_SPTS_SYNCFREE && p->window.use)
+    return solve_window<T, A>(p, b, y, status, st);
   T* yw = (T*)p->ywork;
-  if (algo == SB_SPTS_SYNCFREE || algo == SB_SPTS_HYBRID) {
-    SB_CHECK_CUDA(cudaMemsetAsync(yw, 0xff, sizeof(T) * N, st));
-    SB_CHECK_CUDA(cudaMemsetAsync(p->ticket, 0, sizeof(int), st));
-    if (algo == SB_SPTS_SYNCFREE) {
-      auto k = spts_syncfree_plan_rows<T, A>;
-      k<<<polling_grid((const void*)k, algo, N, p->nlevels), kT, 0, st>>>(
-          p->row_ptr, p->col, (const T*)p->val, N, b, yw, y, p->ticket, limit, status);
-      SB_CHECK_LAUNCH("spts_syncfree_plan_rows");
-    } else {
-      auto k = spts_hybrid_rows<T, A>;
-      k<<<polling_grid((const void*)k, algo, N, p->nlevels), kT, 0, st>>>(
-          p->rrow, p->rcol, (const T*)p->rval, N, p->perm, b, yw, y, p->ticket, limit, status);
-      SB_CHECK_LAUNCH("spts_hybrid_rows");
-    }
+  if (algo == SB_SPTS_LEVEL && p->window.rows <= kLevelBlock) {
+    // the two-round prefetch except for FP32 sums, where the one-round form
+    // measured faster (1M-row random factor, 3470 levels: 6.54 against 7.27
+    // ms; FP64 10.2 -> 9.40 ms with two rounds)
+    constexpr bool two = !(sizeof(T) == 4 && sizeof(A) == 4);
+    spts_level_block<T, A, two><<<1, kLevelBlock, 0, st>>>(
+        p->rrow, p->rcol, (const T*)p->rval, p->level_ptr, p->nlevels, p->perm, b, yw, y);
+    SB_CHECK_LAUNCH("spts_level_block");
     return SB_OK;
   }
-  {
-    // one cooperative launch: a single block of kLevelBlock1 threads when
-    // every level fits in it (no grid barrier), else blocks of kT threads for
-    // the widest level, at most one per SM (fewer blocks make each barrier
-    // cheaper), all of them resident
-    int widest = 0;
-    for (int l = 0; l < p->nlevels; ++l)
-      widest = std::max(widest, p->h_level_ptr[l + 1] - p->h_level_ptr[l]);
-    const int threads = widest <= kLevelBlock1 ? kLevelBlock1 : kT;
-    // the two-round prefetch except for the one-block FP32 form, where the
-    // one-round form measured faster (1M-row random factor, 3470 levels:
-    // 6.54 against 7.27 ms; FP64 10.2 -> 9.40 ms and every grid form
-    // faster with two rounds)
-    const bool two = !(threads == kLevelBlock1 && sizeof(T) == 4 && sizeof(A) == 4);
-    auto k = two ? spts_level_coop<T, A, true> : spts_level_coop<T, A, false>;
-    int per = 0, coop = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)k, threads, 0);
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, p->device);
-    const int blocks =
-        threads == kLevelBlock1
-            ? std::min(1, per * sm_count())
-            : std::min(std::min((widest + kT - 1) / kT, sm_count()), std::max(per, 0) * sm_count());
-    if (coop && blocks >= 1) {
-      unsigned* bar = (unsigned*)(p->ticket + 2);
-      SB_CHECK_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), st));
-      const int* rrow = p->rrow;
-      const int* rcol = p->rcol;
-      const T* rval = (const T*)p->rval;
-      const int* lptr = p->level_ptr;
-      int nl = p->nlevels;
-      const int* perm = p->perm;
-      void* args[] = {(void*)&rrow, (void*)&rcol, (void*)&rval, (void*)&lptr, (void*)&nl,
-                      (void*)&perm, (void*)&b,    (void*)&yw,   (void*)&y,    (void*)&bar,
-                      (void*)&limit, (void*)&status};
-      SB_CHECK_CUDA(
-          cudaLaunchCooperativeKernel((const void*)k, dim3(blocks), dim3(threads), args, 0, st));
-      return SB_OK;
-    }
+  SB_CHECK_CUDA(cudaMemsetAsync(yw, 0xff, sizeof(T) * N, st));
+  SB_CHECK_CUDA(cudaMemsetAsync(p->ticket, 0, sizeof(int), st));
+  if (algo == SB_SPTS_SYNCFREE) {
+    auto k = spts_syncfree_plan_rows<T, A>;
+    k<<<polling_grid((const void*)k, algo, N, p->nlevels), kT, 0, st>>>(
+        p->row_ptr, p->col, (const T*)p->val, N, b, yw, y, p->ticket, limit, status);
+    SB_CHECK_LAUNCH("spts_syncfree_plan_rows");
+  } else {
+    auto k = spts_hybrid_rows<T, A>;
+    k<<<polling_grid((const void*)k, algo, N, p->nlevels), kT, 0, st>>>(
+        p->rrow, p->rcol, (const T*)p->rval, N, p->perm, b, yw, y, p->ticket, limit, status);
+    SB_CHECK_LAUNCH("spts_hybrid_rows");
   }
-  for (int l = 0; l < p->nlevels; ++l) {
-    const int r0 = p->h_level_ptr[l], r1 = p->h_level_ptr[l + 1];
-    if (r1 <= r0) continue;
-    spts_level_rows<T, A><<<grid1(r1 - r0), kT, 0, st>>>(p->rrow, p->rcol, (const T*)p->rval,
-                                                         r0, r1, p->perm, b, yw);
-    SB_CHECK_LAUNCH("spts_level_rows");
-  }
-  scatter_by_perm<T><<<grid1(N), kT, 0, st>>>(yw, p->perm, N, y);
-  SB_CHECK_LAUNCH("scatter_by_perm");
   return SB_OK;
 }
 
@@ -1119,30 +1072,39 @@ static unsigned* noalloc_scratch(int* status) {
 
 using namespace sb;
 
+// A batch's solves run in two branches of one graph, after one copy of the
+// descriptors and counters: the plans with a window layout, each on one block,
+// and the others with ready flags over the whole GPU.  A branch without solves
+// is disabled for the run.
 struct sb_spts_batch {
   int dtype = 0;
   int policy = 0;
   int capacity = 0;
   int device = 0;
-  SptsDesc* h_items = nullptr;   // pinned staging of the descriptors...
-  SptsSched* h_sched = nullptr;  // ...the schedule header...
-  int* h_order = nullptr;        // ...systems by chunk count...
-  long long* h_seg = nullptr;    // ...and segment starts (capacity + 1)
-  SptsDesc* d_items = nullptr;
-  SptsSched* d_sched = nullptr;
-  int* d_order = nullptr;
-  long long* d_seg = nullptr;
-  int* d_tickets = nullptr;      // one chunk counter per item
-  unsigned long long* d_work = nullptr;  // warp-slot counter of the capped grid
+  char* h = nullptr;             // pinned staging of everything below...
+  char* d = nullptr;             // ...and its device copy
+  size_t bytes = 0;
+  // offsets into them
+  size_t items = 0, sched = 0, order = 0, seg = 0, tickets = 0, work = 0;  // ready flags
+  size_t views = 0, moves = 0, count = 0;                                  // windows
   int persistent = 0;            // capped grid: blocks per SM (0 = one warp per slot)
   cudaGraph_t graph_def = nullptr;
   cudaGraphExec_t graph = nullptr;
-  cudaGraphNode_t solve_node = nullptr;
-  cudaKernelNodeParams solve_params = {};
+  cudaGraphNode_t reset_node = nullptr, solve_node = nullptr;
+  cudaGraphNode_t gather_node = nullptr, window_node = nullptr, scatter_node = nullptr;
+  cudaKernelNodeParams solve_params = {}, gather_params = {}, window_params = {},
+                       scatter_params = {};
+  bool flags_on = true, windows_on = true;  // the branches as the graph has them
+  // kernel arguments (device addresses)
+  void *a_items = nullptr, *a_sched = nullptr, *a_order = nullptr, *a_seg = nullptr,
+       *a_tickets = nullptr, *a_work = nullptr, *a_views = nullptr, *a_moves = nullptr,
+       *a_count = nullptr;
+  void* reset_args[2] = {};
   void* solve_args[9] = {};
+  void* move_args[2] = {};
+  void* window_args[3] = {};
   long long limit = 0;
   int* status = nullptr;
-  cudaStream_t capture_stream = nullptr;
   cudaEvent_t done = nullptr;
   bool pending = false;
   int full_per_sm = 1;     // resident blocks per SM of the solve kernel without a cap
@@ -1154,20 +1116,143 @@ struct sb_spts_batch {
 static void spts_batch_release(sb_spts_batch* e) {
   if (e->graph) cudaGraphExecDestroy(e->graph);
   if (e->graph_def) cudaGraphDestroy(e->graph_def);
-  if (e->capture_stream) cudaStreamDestroy(e->capture_stream);
   if (e->done) cudaEventDestroy(e->done);
-  for (void* h : {(void*)e->h_items, (void*)e->h_sched, (void*)e->h_order, (void*)e->h_seg})
-    if (h) cudaFreeHost(h);
-  for (void* d : {(void*)e->d_items, (void*)e->d_sched, (void*)e->d_order, (void*)e->d_seg,
-                  (void*)e->d_tickets, (void*)e->d_work})
-    if (d) cudaFree(d);
+  if (e->h) cudaFreeHost(e->h);
+  if (e->d) cudaFree(e->d);
   delete e;
 }
+
+template <typename T, typename A>
+static const void* window_many(int u) {
+  return u == 4   ? (const void*)win::window_solve_many<T, A, 4>
+         : u == 8 ? (const void*)win::window_solve_many<T, A, 8>
+                  : (const void*)win::window_solve_many<T, A, 16>;
+}
+static const void* window_kernel_for(int dtype, int policy, int u) {
+  if (dtype == SB_F64) return window_many<double, double>(u);
+  if (policy == SB_SPTS_ACC_F64) return window_many<float, double>(u);
+  return window_many<float, float>(u);
+}
+static int window_threads(int dtype, int u) {
+  return 32 * (u == 4   ? win::Warps<float, 4>::n
+               : u == 8 ? (dtype == SB_F64 ? win::Warps<double, 8>::n : win::Warps<float, 8>::n)
+                        : win::Warps<float, 16>::n);
+}
+static_assert(win::Warps<float, 4>::n == win::Warps<double, 4>::n &&
+                  win::Warps<float, 16>::n == win::Warps<double, 16>::n,
+              "window_threads takes these from the FP32 form");
 
 static const void* spts_batch_kernel_for(int dtype, int policy) {
   if (dtype == SB_F64) return (const void*)spts_batch_kernel<double, double>;
   if (policy == SB_SPTS_ACC_F64) return (const void*)spts_batch_kernel<float, double>;
   return (const void*)spts_batch_kernel<float, float>;
+}
+
+// Descriptors and launch shapes of the items whose plans have a window layout
+// (the longest solves first, so that the last blocks to finish are short);
+// returns their number.
+template <typename T>
+static int stage_windows(sb_spts_batch* e, const sb_spts_batch_item* items, int n) {
+  std::vector<std::pair<long long, int>> by_time;  // estimated ns, item
+  int u = 4, window = 0;
+  for (int i = 0; i < n; ++i) {
+    const sb_spts_plan* p = items[i].plan;
+    if (p->N == 0 || !p->window.use) continue;
+    const int pu = win::unroll_of(p->window.kmax);
+    u = std::max(u, pu);
+    window = std::max(window, p->window.window);
+    by_time.push_back({std::max(200LL * p->nlevels, (pu == 4 ? 26LL : pu == 8 ? 45 : 90) *
+                                                        p->ngroups), i});
+  }
+  std::sort(by_time.rbegin(), by_time.rend());
+  const int nw = (int)by_time.size();
+  win::View<T>* views = (win::View<T>*)(e->h + e->views);
+  win::Move<T>* moves = (win::Move<T>*)(e->h + e->moves);
+  long long blocks = 0;
+  for (int k = 0; k < nw; ++k) {
+    const sb_spts_batch_item& it = items[by_time[k].second];
+    T* yw = (T*)(it.work ? it.work : it.plan->ywork);
+    views[k] = window_view<T>(it.plan, yw);
+    moves[k] = {it.plan->perm, (const T*)it.b, yw, (T*)it.y, it.plan->N, (int)blocks};
+    blocks += (it.plan->N + win::kMoveRows - 1) / win::kMoveRows;
+  }
+  *(int*)(e->h + e->count) = nw;
+  e->gather_params.gridDim = e->scatter_params.gridDim =
+      dim3((unsigned)std::max(1LL, blocks));
+  e->window_params.func = const_cast<void*>(window_kernel_for(e->dtype, e->policy, u));
+  e->window_params.blockDim = dim3(window_threads(e->dtype, u));
+  e->window_params.gridDim = dim3(std::max(1, nw));
+  long long smem = win::smem_bytes(window, sizeof(T));
+  // a cap of k blocks per SM: more than 1/(k + 1) of its shared memory each
+  if (e->persistent > 0)
+    smem = std::max(smem, std::min<long long>(win::kSmem, e->smem_per_sm / (e->persistent + 1)));
+  e->window_params.sharedMemBytes = (unsigned)smem;
+  return nw;
+}
+
+// The same for the nf items that are solved with ready flags.
+static int stage_flags(sb_spts_batch* e, const sb_spts_batch_item* items, int n, int nf) {
+  SptsDesc* h_items = (SptsDesc*)(e->h + e->items);
+  int* h_order = (int*)(e->h + e->order);
+  long long* h_seg = (long long*)(e->h + e->seg);
+  SptsSched* h_sched = (SptsSched*)(e->h + e->sched);
+  std::vector<std::pair<int, int>> by_chunks;
+  for (int i = 0; i < n; ++i) {
+    const sb_spts_plan* p = items[i].plan;
+    if (p->N > 0 && p->window.use) continue;
+    const int k = (int)by_chunks.size();
+    SptsDesc& d = h_items[k];
+    d.rrow = p->rrow;
+    d.rcol = p->rcol;
+    d.rval = p->rval;
+    d.perm = p->perm;
+    d.yw = items[i].work ? items[i].work : p->ywork;
+    d.b = items[i].b;
+    d.y = items[i].y;
+    d.N = p->N;
+    d.pad = 0;
+    by_chunks.push_back({(p->N + 31) / 32, k});
+  }
+  std::sort(by_chunks.begin(), by_chunks.end());
+  long long warps = 0;
+  int prev = 0;
+  for (int k = 0; k < nf; ++k) {
+    h_order[k] = by_chunks[k].second;
+    h_seg[k] = warps;
+    warps += (long long)(by_chunks[k].first - prev) * (nf - k);
+    prev = by_chunks[k].first;
+  }
+  h_seg[nf] = warps;
+  h_sched->M = nf;
+  h_sched->warps = warps;
+  const long long per_block = kTB / 32;
+  long long blocks = std::max(1LL, (warps + per_block - 1) / per_block);
+  if (e->persistent > 0)
+    blocks = std::min(blocks, (long long)std::min(e->persistent, e->full_per_sm) * sm_count());
+  SB_REQUIRE(blocks <= 0x7fffffffLL, "sb_spts_batch_run: batch too large");
+  e->solve_params.gridDim = dim3((unsigned)blocks);
+  // Resident blocks per SM: one per 8 systems, up to the occupancy limit.
+  // Every resident warp that holds rows ahead of its system's frontier
+  // polls, so a batch of few systems runs faster with few blocks per SM and
+  // a batch of many with all of them (measured on B200 with FP32 factors: one
+  // of 100k rows 0.95 -> 0.52 ms at one block per SM, 64 of them 0.83 ms at
+  // full occupancy and 1.73 ms at one block per SM).  The cap is dynamic
+  // shared memory that the solve does not use, rounded down to whole KiB, kept
+  // only where the occupancy query confirms at least one block still fits.
+  unsigned smem = 0;
+  const int bps = std::min(e->full_per_sm, std::max(1, (nf + 7) / 8));
+  if (e->persistent == 0 && bps < e->full_per_sm && e->smem_per_sm > 0) {
+    long long want = (long long)e->smem_per_sm / bps - e->smem_reserved;
+    want = std::min<long long>(want, e->smem_optin) / 1024 * 1024;
+    int fit = 0;
+    if (want > 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                        &fit, e->solve_params.func, kTB, (size_t)want) == cudaSuccess &&
+        fit >= 1)
+      smem = (unsigned)want;
+  }
+  e->solve_params.sharedMemBytes = smem;
+  SB_CHECK_CUDA(cudaGraphExecKernelNodeSetParams(e->graph, e->solve_node, &e->solve_params));
+  return SB_OK;
 }
 
 extern "C" {
@@ -1225,75 +1310,103 @@ int sb_spts_batch_create(int dtype, int policy, int32_t capacity, sb_spts_batch*
     spts_batch_release(e);            \
     return r;                         \
   }
-  SB_E(cudaMallocHost(&e->h_items, sizeof(SptsDesc) * capacity));
-  SB_E(cudaMallocHost(&e->h_sched, sizeof(SptsSched)));
-  SB_E(cudaMallocHost(&e->h_order, sizeof(int) * capacity));
-  SB_E(cudaMallocHost(&e->h_seg, sizeof(long long) * (capacity + 1)));
-  SB_E(cudaMalloc(&e->d_items, sizeof(SptsDesc) * capacity));
-  SB_E(cudaMalloc(&e->d_sched, sizeof(SptsSched)));
-  SB_E(cudaMalloc(&e->d_order, sizeof(int) * capacity));
-  SB_E(cudaMalloc(&e->d_seg, sizeof(long long) * (capacity + 1)));
-  SB_E(cudaMalloc(&e->d_tickets, sizeof(int) * capacity));
-  SB_E(cudaMalloc(&e->d_work, sizeof(unsigned long long)));
-  SB_E(cudaStreamCreateWithFlags(&e->capture_stream, cudaStreamNonBlocking));
+  // one block of memory for all descriptors and counters, copied per run
+  const size_t cap = (size_t)capacity;
+  const size_t vsize = dtype == SB_F64 ? sizeof(win::View<double>) : sizeof(win::View<float>);
+  const size_t msize = dtype == SB_F64 ? sizeof(win::Move<double>) : sizeof(win::Move<float>);
+  auto part = [&](size_t bytes) {
+    const size_t at = e->bytes;
+    e->bytes += (bytes + 15) / 16 * 16;
+    return at;
+  };
+  e->items = part(sizeof(SptsDesc) * cap);
+  e->sched = part(sizeof(SptsSched));
+  e->order = part(sizeof(int) * cap);
+  e->seg = part(sizeof(long long) * (cap + 1));
+  e->tickets = part(sizeof(int) * cap);
+  e->work = part(sizeof(unsigned long long));
+  e->views = part(vsize * cap);
+  e->moves = part(msize * cap);
+  e->count = part(sizeof(int));
+  SB_E(cudaMallocHost(&e->h, e->bytes));
+  SB_E(cudaMalloc(&e->d, e->bytes));
   SB_E(cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming));
-  e->h_sched->M = 0;
-  e->h_sched->warps = 0;
+  memset(e->h, 0, e->bytes);
   e->limit = kDefaultSpin;
   e->status = status;
-  // graph: descriptors and schedule (host -> device), tickets to 0, work
-  // vectors to pending, the solve (its grid is set per run)
-  SB_E(cudaStreamBeginCapture(e->capture_stream, cudaStreamCaptureModeThreadLocal));
-  const cudaStream_t cs = e->capture_stream;
-  cudaMemcpyAsync(e->d_items, e->h_items, sizeof(SptsDesc) * capacity, cudaMemcpyHostToDevice, cs);
-  cudaMemcpyAsync(e->d_sched, e->h_sched, sizeof(SptsSched), cudaMemcpyHostToDevice, cs);
-  cudaMemcpyAsync(e->d_order, e->h_order, sizeof(int) * capacity, cudaMemcpyHostToDevice, cs);
-  cudaMemcpyAsync(e->d_seg, e->h_seg, sizeof(long long) * (capacity + 1), cudaMemcpyHostToDevice,
-                  cs);
-  cudaMemsetAsync(e->d_tickets, 0, sizeof(int) * capacity, cs);
-  cudaMemsetAsync(e->d_work, 0, sizeof(unsigned long long), cs);
-  {
-    const void* reset = dtype == SB_F64 ? (const void*)spts_batch_reset<double>
-                                        : (const void*)spts_batch_reset<float>;
-    void* rargs[] = {(void*)&e->d_items, (void*)&e->d_sched};
-    cudaLaunchKernel(reset, dim3(sm_count() * 4), dim3(kT), rargs, 0, cs);
-  }
-  e->solve_args[0] = (void*)&e->d_items;
-  e->solve_args[1] = (void*)&e->d_sched;
-  e->solve_args[2] = (void*)&e->d_order;
-  e->solve_args[3] = (void*)&e->d_seg;
-  e->solve_args[4] = (void*)&e->d_tickets;
-  e->solve_args[5] = (void*)&e->limit;
-  e->solve_args[6] = (void*)&e->status;
-  e->solve_args[7] = (void*)&e->d_work;
-  e->solve_args[8] = (void*)&e->persistent;
+  e->a_items = e->d + e->items;
+  e->a_sched = e->d + e->sched;
+  e->a_order = e->d + e->order;
+  e->a_seg = e->d + e->seg;
+  e->a_tickets = e->d + e->tickets;
+  e->a_work = e->d + e->work;
+  e->a_views = e->d + e->views;
+  e->a_moves = e->d + e->moves;
+  e->a_count = e->d + e->count;
+  const bool f64 = dtype == SB_F64;
+  cudaGraphNode_t copy_node = nullptr;
+  SB_E(cudaGraphCreate(&e->graph_def, 0));
+  SB_E(cudaGraphAddMemcpyNode1D(&copy_node, e->graph_def, nullptr, 0, e->d, e->h, e->bytes,
+                                cudaMemcpyHostToDevice));
+  auto kernel_node = [&](cudaGraphNode_t* node, cudaKernelNodeParams& kp, cudaGraphNode_t after,
+                         const void* func, int blocks, int threads, void** args) {
+    kp.func = const_cast<void*>(func);
+    kp.gridDim = dim3(blocks);
+    kp.blockDim = dim3(threads);
+    kp.sharedMemBytes = 0;
+    kp.kernelParams = args;
+    kp.extra = nullptr;
+    return cudaGraphAddKernelNode(node, e->graph_def, &after, 1, &kp);
+  };
+  // ready flags: work vectors to pending, the solve (its grid is set per run)
   const void* kern = spts_batch_kernel_for(dtype, e->policy);
-  cudaLaunchKernel(kern, dim3(1), dim3(kTB), e->solve_args, 0, cs);
-  SB_E(cudaStreamEndCapture(cs, &e->graph_def));
+  e->reset_args[0] = &e->a_items;
+  e->reset_args[1] = &e->a_sched;
+  e->solve_args[0] = &e->a_items;
+  e->solve_args[1] = &e->a_sched;
+  e->solve_args[2] = &e->a_order;
+  e->solve_args[3] = &e->a_seg;
+  e->solve_args[4] = &e->a_tickets;
+  e->solve_args[5] = &e->limit;
+  e->solve_args[6] = &e->status;
+  e->solve_args[7] = &e->a_work;
+  e->solve_args[8] = &e->persistent;
+  cudaKernelNodeParams reset_params = {};
+  SB_E(kernel_node(&e->reset_node, reset_params, copy_node,
+                   f64 ? (const void*)spts_batch_reset<double>
+                       : (const void*)spts_batch_reset<float>,
+                   sm_count() * 4, kT, e->reset_args));
+  SB_E(kernel_node(&e->solve_node, e->solve_params, e->reset_node, kern, 1, kTB, e->solve_args));
+  // windows: b into level order, the solves, y back into natural order
+  e->move_args[0] = &e->a_moves;
+  e->move_args[1] = &e->a_count;
+  e->window_args[0] = &e->a_views;
+  e->window_args[1] = &e->a_count;
+  e->window_args[2] = &e->status;
+  SB_E(kernel_node(&e->gather_node, e->gather_params, copy_node,
+                   f64 ? (const void*)win::window_move<double, false>
+                       : (const void*)win::window_move<float, false>,
+                   1, 256, e->move_args));
+  SB_E(kernel_node(&e->window_node, e->window_params, e->gather_node,
+                   window_kernel_for(dtype, e->policy, 4), 1, window_threads(dtype, 4),
+                   e->window_args));
+  SB_E(kernel_node(&e->scatter_node, e->scatter_params, e->window_node,
+                   f64 ? (const void*)win::window_move<double, true>
+                       : (const void*)win::window_move<float, true>,
+                   1, 256, e->move_args));
   {
-    size_t nn = 0;
-    SB_E(cudaGraphGetNodes(e->graph_def, nullptr, &nn));
-    std::vector<cudaGraphNode_t> nodes(nn);
-    SB_E(cudaGraphGetNodes(e->graph_def, nodes.data(), &nn));
-    for (cudaGraphNode_t nd : nodes) {
-      cudaGraphNodeType ty;
-      SB_E(cudaGraphNodeGetType(nd, &ty));
-      if (ty != cudaGraphNodeTypeKernel) continue;
-      cudaKernelNodeParams kp = {};
-      SB_E(cudaGraphKernelNodeGetParams(nd, &kp));
-      if (kp.func == kern) {
-        e->solve_node = nd;
-        e->solve_params = kp;
-      }
-    }
-    if (!e->solve_node) {
-      set_error("sb_spts_batch_create: solve node not found in the captured graph");
-      spts_batch_release(e);
-      return SB_ECUDA;
-    }
-    e->solve_params.kernelParams = e->solve_args;
-    e->solve_params.extra = nullptr;
+    // the windows' few large blocks are placed before the other branch's many
+    // small ones, which would keep them off the SMs until they are through
+    int least = 0, greatest = 0;
+    SB_E(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    cudaKernelNodeAttrValue v = {};
+    v.priority = std::max(greatest, least - 1);
+    for (cudaGraphNode_t nd : {e->gather_node, e->window_node})
+      SB_E(cudaGraphKernelNodeSetAttribute(nd, cudaKernelNodeAttributePriority, &v));
   }
+  for (int u : {4, 8, 16})
+    SB_E(cudaFuncSetAttribute(window_kernel_for(dtype, e->policy, u),
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, win::kSmem));
   SB_E(cudaGraphInstantiate(&e->graph, e->graph_def, 0));
   // residency cap of the solve (see sb_spts_batch_run): dynamic shared memory
   // that no solve uses, requested only to limit the blocks per SM
@@ -1361,69 +1474,36 @@ int sb_spts_batch_run(sb_spts_batch* e, const sb_spts_batch_item* items, int32_t
       SB_REQUIRE(ps[i] != ps[i - 1],
                  "sb_spts_batch_run: a plan appears twice in one batch with its own work vector");
   }
-  // the pinned staging buffers are read by the previous run's first nodes
+  // the pinned staging buffer is read by the previous run's first node
   if (e->pending) SB_CHECK_CUDA(cudaEventSynchronize(e->done));
   cudaStream_t st = as_stream(stream);
-  std::vector<std::pair<int, int>> by_chunks(n);
-  for (int i = 0; i < n; ++i) {
-    sb_spts_plan* p = items[i].plan;
-    SptsDesc& d = e->h_items[i];
-    d.rrow = p->rrow;
-    d.rcol = p->rcol;
-    d.rval = p->rval;
-    d.perm = p->perm;
-    d.yw = items[i].work ? items[i].work : p->ywork;
-    d.b = items[i].b;
-    d.y = items[i].y;
-    d.N = p->N;
-    d.pad = 0;
-    by_chunks[i] = {(p->N + 31) / 32, i};
+  const int nw = e->dtype == SB_F64 ? stage_windows<double>(e, items, n)
+                                    : stage_windows<float>(e, items, n);
+  const int nf = n - nw;
+  if (nw > 0) {
+    SB_CHECK_CUDA(cudaGraphExecKernelNodeSetParams(e->graph, e->gather_node, &e->gather_params));
+    SB_CHECK_CUDA(cudaGraphExecKernelNodeSetParams(e->graph, e->window_node, &e->window_params));
+    SB_CHECK_CUDA(cudaGraphExecKernelNodeSetParams(e->graph, e->scatter_node, &e->scatter_params));
   }
-  std::sort(by_chunks.begin(), by_chunks.end());
-  long long warps = 0;
-  int prev = 0;
-  for (int k = 0; k < n; ++k) {
-    e->h_order[k] = by_chunks[k].second;
-    e->h_seg[k] = warps;
-    warps += (long long)(by_chunks[k].first - prev) * (n - k);
-    prev = by_chunks[k].first;
+  if (nf > 0) {
+    const int r = stage_flags(e, items, n, nf);
+    if (r) return r;
   }
-  e->h_seg[n] = warps;
-  e->h_sched->M = n;
-  e->h_sched->warps = warps;
-  const long long per_block = kTB / 32;
-  long long blocks = std::max(1LL, (warps + per_block - 1) / per_block);
-  if (e->persistent > 0)
-    blocks = std::min(blocks, (long long)std::min(e->persistent, e->full_per_sm) * sm_count());
-  SB_REQUIRE(blocks <= 0x7fffffffLL, "sb_spts_batch_run: batch too large");
-  e->solve_params.gridDim = dim3((unsigned)blocks);
-  // Resident blocks per SM: one per 8 systems, up to the occupancy limit.
-  // Every resident warp that holds rows ahead of its system's frontier
-  // polls, so a batch of few systems runs faster with few blocks per SM and
-  // a batch of many with all of them (measured on B200: one 100k-row factor
-  // 0.95 -> 0.52 ms at one block per SM, 64 of them 0.83 ms at full
-  // occupancy and 1.73 ms at one block per SM).  The cap is dynamic shared
-  // memory that the solve does not use, rounded down to whole KiB, kept only
-  // where the occupancy query confirms at least one block still fits.
-  unsigned smem = 0;
-  const int bps = std::min(e->full_per_sm, std::max(1, (n + 7) / 8));
-  if (e->persistent == 0 && bps < e->full_per_sm && e->smem_per_sm > 0) {
-    long long want = (long long)e->smem_per_sm / bps - e->smem_reserved;
-    want = std::min<long long>(want, e->smem_optin) / 1024 * 1024;
-    int fit = 0;
-    if (want > 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                        &fit, e->solve_params.func, kTB, (size_t)want) == cudaSuccess &&
-        fit >= 1)
-      smem = (unsigned)want;
+  if ((nw > 0) != e->windows_on) {
+    for (cudaGraphNode_t nd : {e->gather_node, e->window_node, e->scatter_node})
+      SB_CHECK_CUDA(cudaGraphNodeSetEnabled(e->graph, nd, nw > 0));
+    e->windows_on = nw > 0;
   }
-  e->solve_params.sharedMemBytes = smem;
-  SB_CHECK_CUDA(cudaGraphExecKernelNodeSetParams(e->graph, e->solve_node, &e->solve_params));
+  if ((nf > 0) != e->flags_on) {
+    for (cudaGraphNode_t nd : {e->reset_node, e->solve_node})
+      SB_CHECK_CUDA(cudaGraphNodeSetEnabled(e->graph, nd, nf > 0));
+    e->flags_on = nf > 0;
+  }
   SB_CHECK_CUDA(cudaGraphLaunch(e->graph, st));
   SB_CHECK_CUDA(cudaEventRecord(e->done, st));
   e->pending = true;
   return SB_OK;
 }
-
 
 int sb_spts_syncfree_csr_noalloc(int dtype, const int32_t* row_ptr, const int32_t* col,
                                  const void* val, int32_t N, const void* b, void* y,
@@ -1557,6 +1637,19 @@ int sb_spts_plan_reordered(const sb_spts_plan* plan, int32_t* row_ptr, int32_t* 
   if (row_ptr)
     SB_CHECK_CUDA(cudaMemcpyAsync(row_ptr, plan->rrow, sizeof(int) * ((size_t)plan->N + 1),
                                   cudaMemcpyDeviceToDevice, st));
+  if (plan->window.use && (col || val)) {
+    const unsigned g = grid1(32LL * plan->ngroups);
+    if (plan->dtype == SB_F64)
+      win::window_to_csr<double><<<g, kT, 0, st>>>(plan->rrow, plan->level_ptr, plan->groups,
+                                                   plan->ngroups, plan->window.window,
+                                                   plan->records, col, (double*)val);
+    else
+      win::window_to_csr<float><<<g, kT, 0, st>>>(plan->rrow, plan->level_ptr, plan->groups,
+                                                  plan->ngroups, plan->window.window,
+                                                  plan->records, col, (float*)val);
+    SB_CHECK_LAUNCH("window_to_csr");
+    return SB_OK;
+  }
   if (col)
     SB_CHECK_CUDA(cudaMemcpyAsync(col, plan->rcol, sizeof(int) * (size_t)plan->nnz,
                                   cudaMemcpyDeviceToDevice, st));
