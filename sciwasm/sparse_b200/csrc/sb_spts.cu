@@ -9,8 +9,9 @@
 // reordered CSR with columns relabelled by order[] is built.  All integer
 // outputs are bit-exact.  Levels are computed by one thread per row, rows
 // handed out in increasing order through a warp ticket so that every row a
-// thread waits for has already been claimed by a running warp; each wait is
-// an acquire load with a clock bound.
+// thread waits for has already been claimed by a running warp (or, for rows that
+// read rows shortly before them, by one cluster in a fixed order); each wait is
+// bounded.
 //
 // Solves (one thread per row, storage order, separately rounded mul/add, so
 // the results are bit-identical to the reference's row kernels):
@@ -59,7 +60,6 @@ struct sb_spts_plan {
   int* ticket = nullptr;
   // window layout (in the memory of rcol and rval, which are then not stored)
   sb::win::Info window = {};
-  int ngroups = 0;
   int4* groups = nullptr;
   char* records = nullptr;
   std::vector<void*> owned;
@@ -233,60 +233,330 @@ __device__ __forceinline__ A dot_published(const int* __restrict__ col, const T*
 
 // ------------------------------------------------------------ analysis
 
-// flags[0] = 1 unless every row is non-empty, ends with its diagonal and has
-// all other columns in [0, i) (the structure the solves require).
-__global__ void lower_check(const int* __restrict__ row_ptr, const int* __restrict__ col, int N,
-                            int* __restrict__ flags) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  const int s = row_ptr[i], e = row_ptr[i + 1];
-  bool ok = e > s && col[e - 1] == i;
-  for (int j = s; ok && j < e - 1; ++j) ok = col[j] >= 0 && col[j] < i;
-  if (!ok) flags[0] = 1;
-}
+// What one pass over the structure tells: lower_bad = 1 unless every row is
+// non-empty, ends with its diagonal and has all other columns in [0, i) (the
+// structure the solves require); and how many rows read a row less than
+// kNearRows before them, and one less than kClusterRows before them.
+constexpr int kNearRows = 32;       // the rows of a warp
+constexpr int kClusterBlocks = 8;   // the largest portable cluster
+constexpr int kClusterThreads = 256;
+constexpr int kClusterRows = kClusterBlocks * kClusterThreads;
 
-__global__ void level_kernel(const int* __restrict__ row_ptr, const int* __restrict__ col, int N,
-                             int* level, int* __restrict__ ticket, long long limit,
-                             int* __restrict__ status) {
-  while (true) {
-    const int base = next_rows(ticket);
-    if (base >= N) return;
-    const int i = base + (threadIdx.x & 31);
-    if (i < N) {
-      const int s = row_ptr[i], e = row_ptr[i + 1];
-      int lv;
-      if (e - s == 1) {
-        lv = 0;
-      } else {
-        int m = 0;
-        for (int j0 = s; j0 < e - 1; j0 += kG) {
-          int c[kG], v[kG];
-#pragma unroll
-          for (int k = 0; k < kG; ++k) {
-            // columns outside [0, i) read as level 0 (row 0's slot, never pending)
-            const int cc = (j0 + k < e - 1) ? col[j0 + k] : -1;
-            c[k] = (cc >= 0 && cc < i) ? cc : -1;
-          }
-#pragma unroll
-          for (int k = 0; k < kG; ++k) v[k] = c[k] >= 0 ? ld_relaxed(level + c[k]) : 0;
-          wait_group(level, c, v, kG, limit, status);
-#pragma unroll
-          for (int k = 0; k < kG; ++k) m = v[k] > m ? v[k] : m;
-        }
-        lv = 1 + m;
-      }
-      st_relaxed(level + i, lv);
+struct Shape {
+  int lower_bad;
+  int top;          // the highest level
+  int near_rows;    // rows with a dependency in the kNearRows before
+  int reach_rows;   // rows with one in the kClusterRows before
+  int ticket;       // rows handed out
+  int status;       // a wait's timeout
+};
+
+__global__ void shape_check(const int* __restrict__ row_ptr, const int* __restrict__ col, int N,
+                            Shape* __restrict__ shape) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  bool ok = true;
+  int last = -1;  // the nearest row before i that it reads
+  if (i < N) {
+    const int s = row_ptr[i], e = row_ptr[i + 1];
+    ok = e > s && col[e - 1] == i;
+    for (int j = s; j < e - 1; ++j) {
+      const int c = col[j];
+      ok = ok && c >= 0 && c < i;
+      if (c < i) last = max(last, c);
     }
+  }
+  const int near = __syncthreads_count(last >= 0 && i - last < kNearRows);
+  const int reach = __syncthreads_count(last >= 0 && i - last < kClusterRows);
+  const int bad = __syncthreads_or(!ok);
+  if (threadIdx.x == 0) {
+    if (near) atomicAdd(&shape->near_rows, near);
+    if (reach) atomicAdd(&shape->reach_rows, reach);
+    if (bad) shape->lower_bad = 1;
   }
 }
 
-__global__ void max_kernel(const int* __restrict__ a, int n, int* __restrict__ out) {
-  int m = 0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    m = max(m, a[i]);
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+// Columns of up to kG entries from s on of row i, but its last (-1: none, or
+// outside [0, i), which reads as level 0).
+__device__ __forceinline__ void row_columns(const int* __restrict__ col, int i, int s, int e,
+                                            int (&c)[kG]) {
+#pragma unroll
+  for (int k = 0; k < kG; ++k) {
+    const int cc = s + k < e - 1 ? __ldg(col + s + k) : -1;
+    c[k] = cc < i ? cc : -1;
+  }
+}
+
+// Entries of a lane's row that name rows of its own warp (rows base ..
+// base + 31, one per lane) take their levels from registers: chains inside a
+// warp (a stencil in natural order reads row i - 1) cost a shuffle a row
+// instead of a trip through L2.  lv: a lane's level, -1 until known; inner: the
+// entries waited for.
+__device__ __forceinline__ void take_inner(const int (&c)[kG], int base, int lv, unsigned& inner,
+                                           int& m) {
+  const unsigned any = __reduce_or_sync(0xffffffffu, inner);
+#pragma unroll
+  for (int k = 0; k < kG; ++k)
+    if (any & (1u << k)) {
+      const int v = __shfl_sync(0xffffffffu, lv, c[k] - base);
+      if ((inner & (1u << k)) && v >= 0) {
+        m = max(m, v);
+        inner &= ~(1u << k);
+      }
+    }
+}
+
+// One warp per 32 rows, in order (tickets).  Before the chains inside a warp
+// went through registers, 3-D Laplacians took 0.56 / 2.2 / 4.9 ms (64^3 /
+// 100^3 / 128^3, analysis in all, on B200), now 0.37 / 1.06 / 2.2, 100k rows
+// with band 50 18.1, now 8.6.  More than `few` blocks (two per SM) pay where
+// such chains hold rows back (0.43 -> 0.37 ms on 64^3) and cost where rows only
+// wait for far ones (300k rows, band 100k: 0.41 -> 0.63 ms), so the others leave
+// unless half the rows read one of the kNearRows before them.
+__global__ void level_kernel(const int* __restrict__ row_ptr, const int* __restrict__ col, int N,
+                             int* level, Shape* __restrict__ shape, int few, long long limit) {
+  if ((int)blockIdx.x >= few && 2LL * shape->near_rows < N) return;
+  const int lane = threadIdx.x & 31;
+  int top = 0;
+  while (true) {
+    const int base = next_rows(&shape->ticket);
+    if (base >= N) break;
+    const int i = base + lane;
+    int s = 0, e = 1, j0 = 0, m = 0, lv = i < N ? -1 : 0, spins = 0;
+    int c[kG];
+    unsigned outer = 0, inner = 0;
+    if (i < N) {
+      j0 = s = row_ptr[i];
+      e = row_ptr[i + 1];
+    }
+    row_columns(col, i, s, e, c);
+#pragma unroll
+    for (int k = 0; k < kG; ++k)
+      if (c[k] >= base) inner |= 1u << k;
+      else if (c[k] >= 0) outer |= 1u << k;
+    unsigned ns = SB_SPTS_SLEEP_MIN_NS;
+    long long t0 = 0;
+    while (true) {
+      if (outer) {
+        int v[kG];
+#pragma unroll
+        for (int k = 0; k < kG; ++k)
+          if (outer & (1u << k)) v[k] = ld_relaxed(level + c[k]);
+#pragma unroll
+        for (int k = 0; k < kG; ++k)
+          if ((outer & (1u << k)) && v[k] >= 0) {
+            m = max(m, v[k]);
+            outer &= ~(1u << k);
+          }
+      }
+      bool known;
+      do {
+        known = false;
+        if (lv < 0 && !(outer | inner)) {
+          j0 += kG;
+          if (j0 < e - 1) {  // a long row's next entries
+            row_columns(col, i, j0, e, c);
+#pragma unroll
+            for (int k = 0; k < kG; ++k)
+              if (c[k] >= base) inner |= 1u << k;
+              else if (c[k] >= 0) outer |= 1u << k;
+            known = inner != 0;  // take what is known already
+          } else {
+            lv = e - s == 1 ? 0 : 1 + m;
+            st_relaxed(level + i, lv);
+            known = true;
+          }
+        }
+        known = __any_sync(0xffffffffu, known);
+        if (known) take_inner(c, base, lv, inner, m);
+      } while (known);
+      if (!__any_sync(0xffffffffu, lv < 0)) break;
+      if (++spins > 1) {
+        __nanosleep(ns);
+        ns = ns < SB_SPTS_SLEEP_MAX_NS ? 2 * ns : ns;
+        if ((spins & 255) == 0) {
+          if (t0 == 0) t0 = clock64();
+          if (clock64() - t0 > limit || *(volatile const int*)&shape->status) {
+            // the call fails; the rows that waited end at a level of their own
+            atomicExch(&shape->status, SB_DEV_TIMEOUT_DEP);
+            if (lv < 0) st_relaxed(level + i, lv = 0);
+            outer = inner = 0;
+          }
+        }
+      }
+    }
+    top = max(top, lv);
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0 && top > 0) atomicMax(&shape->top, top);
+}
+
+// The same on one cluster of kClusterBlocks blocks, for factors whose rows
+// mostly read rows a little before them: each block keeps the levels of the
+// last kRing rows in its shared memory, and a row's level is stored into every
+// block's ring, so a dependency costs a store across the cluster and a
+// shared-memory poll (0.55 us) rather than two trips through L2 (1.3 us).
+// A ring entry is one 64-bit word, the row (plus 1) above its level, so a
+// reader can tell its row's entry from an older one (poll on) or a newer one
+// (the entry is gone: read the level's global word, -1 until it is there).
+// Stores of different blocks to one slot may land in either order, which could
+// leave an older row's entry for good, so a long wait turns to global memory
+// as well; no wait depends on the ring alone.  Consecutive 32-row chunks go to
+// different blocks; the lowest unfinished row always has its warp running and
+// its dependencies published, and a row publishes its level while others of
+// its warp still wait.
+//
+// It runs where at least 3/4 of the rows read one of the kClusterRows before
+// them (those in flight: with fewer, rows far apart are independent and the
+// whole GPU is the better place) and less than half read one of the kNearRows
+// before them (chains inside a warp: a stencil in natural order); otherwise it
+// leaves the ticket at 0 and level_kernel takes all rows.  Analysis in all,
+// level_kernel alone -> with this one, on B200: 1M-row random factor with band
+// 5000 4.7 -> 2.3 ms, 100k rows with band 500 2.3 -> 1.9; without the rule a 3-D
+// Laplacian 64^3 would take 2.3 instead of 0.4, 300k rows with band 100k 0.73
+// instead of 0.41.  Fewer or more blocks or warps, sleeping between polls, rows
+// spread over the warps and one block sweeping over 1024 rows at a time were
+// slower.
+constexpr int kRing = 16384;  // entries: 128 KB
+
+__device__ __forceinline__ unsigned long long ld_entry(uint32_t a) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_entry(uint32_t a, unsigned long long v) {
+  asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t peer_address(uint32_t a, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::
+                   : "memory");
+}
+
+// Which of a row's entries lie in the ring, and which are too far back for it.
+__device__ __forceinline__ void row_waits(const int (&c)[kG], int i, unsigned& pend,
+                                          unsigned& far) {
+#pragma unroll
+  for (int k = 0; k < kG; ++k)
+    if (c[k] >= 0) {
+      if (i - c[k] < kRing) pend |= 1u << k;
+      else far |= 1u << k;
+    }
+}
+
+__global__ void __launch_bounds__(kClusterThreads, 1)
+    level_cluster_kernel(const int* __restrict__ row_ptr, const int* __restrict__ col, int N,
+                         int* level, Shape* __restrict__ shape, long long limit) {
+  extern __shared__ __align__(16) unsigned long long ring[];
+  int* status = &shape->status;
+  int top = 0;
+  if (4LL * shape->reach_rows < 3LL * N || 2LL * shape->near_rows >= N) return;
+  for (int k = threadIdx.x; k < kRing; k += kClusterThreads) ring[k] = 0;
+  const uint32_t own = smem_u32(ring);
+  uint32_t peer[kClusterBlocks];
+#pragma unroll
+  for (int r = 0; r < kClusterBlocks; ++r) peer[r] = peer_address(own, r);
+  cluster_barrier();
+  const int lane = threadIdx.x & 31;
+  constexpr int step = kClusterRows;
+  int i = 32 * ((threadIdx.x >> 5) * kClusterBlocks + (int)blockIdx.x) + lane;
+  int s = 0, e = 0, s1 = 0, e1 = 0;
+  int c[kG], c1[kG];
+#pragma unroll
+  for (int k = 0; k < kG; ++k) c[k] = c1[k] = -1;
+  if (i < N) {
+    s = __ldg(row_ptr + i);
+    e = __ldg(row_ptr + i + 1);
+    row_columns(col, i, s, e, c);
+  }
+  if (i + (long long)step < N) {
+    s1 = __ldg(row_ptr + i + step);
+    e1 = __ldg(row_ptr + i + step + 1);
+  }
+  for (long long first = i - lane; first < N; first += step) {
+    // ahead: the next row's columns and the bounds of the row after it
+    const bool next = i + (long long)step < N, second = i + 2LL * step < N;
+    if (next) row_columns(col, i + step, s1, e1, c1);
+    int s2 = 0, e2 = 0;
+    if (second) {
+      s2 = __ldg(row_ptr + i + 2 * step);
+      e2 = __ldg(row_ptr + i + 2 * step + 1);
+    }
+    bool waiting = first + lane < N;
+    int m = 0, j0 = s, spins = 0;
+    unsigned pend = 0, far = 0;
+    row_waits(c, i, pend, far);
+    long long t0 = 0;
+    while (__any_sync(0xffffffffu, waiting)) {
+      if (waiting) {
+        unsigned long long w[kG];
+#pragma unroll
+        for (int k = 0; k < kG; ++k)
+          if (pend & (1u << k)) w[k] = ld_entry(own + (uint32_t)(c[k] & (kRing - 1)) * 8u);
+#pragma unroll
+        for (int k = 0; k < kG; ++k)
+          if (pend & (1u << k)) {
+            const int ahead = (int)(w[k] >> 32) - (c[k] + 1);
+            if (ahead == 0) m = max(m, (int)w[k]);
+            if (ahead >= 0) pend &= ~(1u << k);
+            if (ahead > 0) far |= 1u << k;
+          }
+        const bool long_wait = (++spins & 63) == 0;
+        if (far || long_wait) {
+          const unsigned ask = far | (long_wait ? pend : 0u);
+#pragma unroll
+          for (int k = 0; k < kG; ++k)
+            if (ask & (1u << k)) {
+              const int v = ld_relaxed(level + c[k]);
+              if (v >= 0) {
+                m = max(m, v);
+                far &= ~(1u << k);
+                pend &= ~(1u << k);
+              }
+            }
+        }
+        if (!(pend | far)) {
+          j0 += kG;
+          if (j0 < e - 1) {  // a long row's next entries
+            row_columns(col, i, j0, e, c);
+            row_waits(c, i, pend, far);
+          } else {
+            const int lv = e - s == 1 ? 0 : 1 + m;
+            const unsigned long long v =
+                (unsigned long long)(unsigned)(i + 1) << 32 | (unsigned)lv;
+            const uint32_t o = (uint32_t)(i & (kRing - 1)) * 8u;
+#pragma unroll
+            for (int r = 0; r < kClusterBlocks; ++r) st_entry(peer[r] + o, v);
+            st_relaxed(level + i, lv);
+            top = max(top, lv);
+            waiting = false;
+          }
+        } else if ((spins & 1023) == 0) {
+          if (t0 == 0) t0 = clock64();
+          if (clock64() - t0 > limit || *(volatile const int*)status) {
+            atomicExch(status, SB_DEV_TIMEOUT_DEP);
+            st_relaxed(level + i, 0);  // the call fails; the kernel ends
+            waiting = false;
+          }
+        }
+      }
+    }
+    s = s1;
+    e = e1;
+    s1 = s2;
+    e1 = e2;
+    i = next ? i + step : i;
+#pragma unroll
+    for (int k = 0; k < kG; ++k) c[k] = next ? c1[k] : -1;
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0 && top > 0) atomicMax(&shape->top, top);
+  cluster_barrier();  // no block leaves while others still store into its ring
+  if (blockIdx.x == 0 && threadIdx.x == 0) shape->ticket = N;
 }
 
 __global__ void level_hist(const int* __restrict__ level, int N, int* __restrict__ counts) {
@@ -746,12 +1016,10 @@ static int resident_grid(const void* kern) {
 //    CTAs, 9.5 ms at 148 on 128^3) and one CTA per SM when they are narrow
 //    (288 rows per level: 9.5 -> 4.4 ms).
 // Grid of the natural-order polling kernels that run without level
-// information (the analysis itself and the sync-free solve on caller
-// arrays): two CTAs per SM.  Measured on B200 against the resident grid
-// (analysis / caller-array sync-free, ms): 3-D Laplacian 64^3 3.35 -> 3.16 /
-// 1.51 -> 1.50; 128^3 8.58 -> 8.15 / 15.2 -> 15.4; 1M-row random factor
-// 18.1 -> 8.1 / 41.0 -> 25.9; band-50 1M 425 -> 224 / 2048 -> 1368;
-// bidiagonal 100k 122 -> 81 / 265 -> 259.  One CTA per SM was faster still on
+// information (the sync-free solve on caller arrays): two CTAs per SM.
+// Measured on B200 against the resident grid (ms): 3-D Laplacian 64^3 1.51 ->
+// 1.50; 128^3 15.2 -> 15.4; 1M-row random factor 41.0 -> 25.9; band-50 1M
+// 2048 -> 1368; bidiagonal 100k 265 -> 259.  One CTA per SM was faster still on
 // the narrow factors and 30-50% slower on the Laplacians.
 static int natural_order_grid(const void* kern) {
   return std::min(resident_grid(kern), 2 * sm_count());
@@ -775,6 +1043,26 @@ static void plan_release(sb_spts_plan* p) {
   if (p->ev[0]) cudaEventDestroy(p->ev[0]);
   if (p->ev[1]) cudaEventDestroy(p->ev[1]);
   p->ev[0] = p->ev[1] = nullptr;
+}
+
+static int launch_level_cluster(const sb_spts_plan* p, Shape* shape, cudaStream_t st) {
+  const size_t smem = sizeof(unsigned long long) * kRing;
+  SB_CHECK_CUDA(cudaFuncSetAttribute((const void*)level_cluster_kernel,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kClusterBlocks);
+  cfg.blockDim = dim3(kClusterThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kClusterBlocks;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  SB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, level_cluster_kernel, p->row_ptr, p->col, p->N, p->level,
+                                   shape, (long long)kDefaultSpin));
+  return SB_OK;
 }
 
 template <typename T>
@@ -812,38 +1100,28 @@ static int analyze_impl(sb_spts_plan* p, cudaStream_t st) {
     SB_CHECK_CUDA(cudaEventCreate(&p->ev[0]));
     SB_CHECK_CUDA(cudaEventCreate(&p->ev[1]));
   }
-  int* status = device_status_word();
-  if (!status) {
-    set_error("sb_spts_analyze: device status word unavailable");
-    return SB_ENOMEM;
-  }
   SB_CHECK_CUDA(cudaEventRecord(p->ev[0], st));
-  int* tmp = nullptr;  // [0] lower-check flag, [1] max level
-  if ((r = scratch_alloc((void**)&tmp, 4 * sizeof(int), st))) return r;
-  SB_CHECK_CUDA(cudaMemsetAsync(tmp, 0, 4 * sizeof(int), st));
-  lower_check<<<grid1(N), kT, 0, st>>>(p->row_ptr, p->col, N, tmp);
-  SB_CHECK_LAUNCH("lower_check");
+  Shape* shape = nullptr;
+  if ((r = scratch_alloc((void**)&shape, sizeof(Shape), st))) return r;
+  SB_CHECK_CUDA(cudaMemsetAsync(shape, 0, sizeof(Shape), st));
+  shape_check<<<grid1(N), kT, 0, st>>>(p->row_ptr, p->col, N, shape);
+  SB_CHECK_LAUNCH("shape_check");
   SB_CHECK_CUDA(cudaMemsetAsync(p->level, 0xff, sizeof(int) * N, st));
-  SB_CHECK_CUDA(cudaMemsetAsync(p->ticket, 0, sizeof(int), st));
-  level_kernel<<<natural_order_grid((const void*)level_kernel), kT, 0, st>>>(
-      p->row_ptr, p->col, N, p->level, p->ticket, kDefaultSpin, status);
+  // (a few thousand rows leave the cluster nothing to gain)
+  if (N >= 4 * kClusterRows && (r = launch_level_cluster(p, shape, st))) return r;
+  level_kernel<<<std::min(resident_grid((const void*)level_kernel), 4 * sm_count()), kT, 0, st>>>(
+      p->row_ptr, p->col, N, p->level, shape, 2 * sm_count(), kDefaultSpin);
   SB_CHECK_LAUNCH("level_kernel");
-  max_kernel<<<std::min<unsigned>(grid1(N), (unsigned)sm_count() * 4), kT, 0, st>>>(p->level, N,
-                                                                                    tmp + 1);
-  SB_CHECK_LAUNCH("max_kernel");
-  int h[2] = {0, 0};
-  SB_CHECK_CUDA(cudaMemcpyAsync(h, tmp, sizeof(h), cudaMemcpyDeviceToHost, st));
-  int dstat = 0;
-  SB_CHECK_CUDA(cudaMemcpyAsync(&dstat, status, sizeof(int), cudaMemcpyDeviceToHost, st));
+  Shape h = {};
+  SB_CHECK_CUDA(cudaMemcpyAsync(&h, shape, sizeof(h), cudaMemcpyDeviceToHost, st));
   SB_CHECK_CUDA(cudaStreamSynchronize(st));
-  scratch_free(tmp, st);
-  if (dstat) {
-    cudaMemsetAsync(status, 0, sizeof(int), st);
+  scratch_free(shape, st);
+  if (h.status) {
     set_error("sb_spts_analyze: a level dependency wait timed out");
     return SB_ETIMEOUT;
   }
-  p->solvable = h[0] ? 0 : 1;
-  p->nlevels = N ? h[1] + 1 : 0;
+  p->solvable = h.lower_bad ? 0 : 1;
+  p->nlevels = N ? h.top + 1 : 0;
   const int L = p->nlevels;
   // level_ptr = exclusive scan of the per-level counts
   SB_CHECK_CUDA(cudaMemsetAsync(p->level_ptr, 0, sizeof(int) * ((size_t)L + 1), st));
@@ -892,8 +1170,8 @@ static int analyze_impl(sb_spts_plan* p, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(gstart, 0, lb + 2 * gb + 256, st);
   if (e != cudaSuccess) r = cuda_status(e, "sb_spts_analyze");
   if (!r) {
-    win::window_reach<<<grid1(N), kT, 0, st>>>(p->row_ptr, p->col, p->level, p->level_ptr, N, info);
-    win::window_level_groups<<<grid1(L + 1), kT, 0, st>>>(p->level_ptr, L, gstart, info);
+    win::window_reach<<<grid1((long long)N + 1), kT, 0, st>>>(p->row_ptr, p->col, p->level,
+                                                              p->level_ptr, N, L, gstart, info);
     e = cudaGetLastError();
     if (e != cudaSuccess) r = cuda_status(e, "window_reach");
     if (!r) r = prim::exclusive_scan(gstart, gstart, L + 1, st);
@@ -914,16 +1192,11 @@ static int analyze_impl(sb_spts_plan* p, cudaStream_t st) {
   if (!r) {
     // row lengths in level order, scanned into rrow
     int* lens = (int*)rb.k[0];
-    win::window_lengths<<<grid1(N), kT, 0, st>>>(p->row_ptr, p->perm, p->level, p->level_ptr,
+    win::window_lengths<<<grid1((long long)N + 1), kT, 0, st>>>(p->row_ptr, p->perm, p->level, p->level_ptr,
                                                  gstart, N, lens, groups, glen);
     e = cudaGetLastError();
     if (e != cudaSuccess) r = cuda_status(e, "window_lengths");
-    if (!r) r = prim::exclusive_scan(lens, p->rrow, N, st);
-    if (!r) {
-      const int nz = (int)nnz;
-      e = cudaMemcpyAsync(p->rrow + N, &nz, sizeof(int), cudaMemcpyHostToDevice, st);
-      if (e != cudaSuccess) r = cuda_status(e, "rrow");
-    }
+    if (!r) r = prim::exclusive_scan(lens, p->rrow, (long long)N + 1, st);
     if (!r && groups) {
       win::window_sizes<<<grid1(gmax + 1), kT, 0, st>>>(groups, glen, gmax, gstart + L,
                                                         sizeof(T), gbase, info);
@@ -931,11 +1204,9 @@ static int analyze_impl(sb_spts_plan* p, cudaStream_t st) {
       if (e != cudaSuccess) r = cuda_status(e, "window_sizes");
       if (!r) r = prim::exclusive_scan(gbase, gbase, gmax + 1, st);
       if (!r) {
-        win::window_decide<<<1, 1, 0, st>>>(gbase + gmax, gstart + L, L, cap, sizeof(T),
-                                             h[0] == 0, info);
         win::window_fill<T><<<grid1(N), kT, 0, st>>>(
             p->row_ptr, p->col, (const T*)p->val, p->perm, p->order, p->level, p->level_ptr, gstart,
-            glen, gbase, N, info, groups, p->records);
+            glen, gbase, N, L, gmax, cap, h.lower_bad == 0, info, groups, p->records);
         e = cudaGetLastError();
         if (e != cudaSuccess) r = cuda_status(e, "window_fill");
       }
@@ -951,8 +1222,6 @@ static int analyze_impl(sb_spts_plan* p, cudaStream_t st) {
     e = cudaEventRecord(p->ev[1], st);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(&p->window, info, sizeof(win::Info), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(&p->ngroups, gstart + L, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = cudaEventElapsedTime(&p->analysis_ms, p->ev[0], p->ev[1]);
     if (e != cudaSuccess) r = cuda_status(e, "sb_spts_analyze");
@@ -963,7 +1232,7 @@ static int analyze_impl(sb_spts_plan* p, cudaStream_t st) {
 
 template <typename T>
 static win::View<T> window_view(const sb_spts_plan* p, T* yw) {
-  return {p->groups,         p->records,     yw, p->ngroups, p->window.window,
+  return {p->groups,         p->records,     yw, p->window.ngroups, p->window.window,
           p->window.kmax, p->window.widest};
 }
 
@@ -1162,7 +1431,7 @@ static int stage_windows(sb_spts_batch* e, const sb_spts_batch_item* items, int 
     u = std::max(u, pu);
     window = std::max(window, p->window.window);
     by_time.push_back({std::max(200LL * p->nlevels, (pu == 4 ? 26LL : pu == 8 ? 45 : 90) *
-                                                        p->ngroups), i});
+                                                        p->window.ngroups), i});
   }
   std::sort(by_time.rbegin(), by_time.rend());
   const int nw = (int)by_time.size();
@@ -1638,14 +1907,14 @@ int sb_spts_plan_reordered(const sb_spts_plan* plan, int32_t* row_ptr, int32_t* 
     SB_CHECK_CUDA(cudaMemcpyAsync(row_ptr, plan->rrow, sizeof(int) * ((size_t)plan->N + 1),
                                   cudaMemcpyDeviceToDevice, st));
   if (plan->window.use && (col || val)) {
-    const unsigned g = grid1(32LL * plan->ngroups);
+    const unsigned g = grid1(32LL * plan->window.ngroups);
     if (plan->dtype == SB_F64)
       win::window_to_csr<double><<<g, kT, 0, st>>>(plan->rrow, plan->level_ptr, plan->groups,
-                                                   plan->ngroups, plan->window.window,
+                                                   plan->window.ngroups, plan->window.window,
                                                    plan->records, col, (double*)val);
     else
       win::window_to_csr<float><<<g, kT, 0, st>>>(plan->rrow, plan->level_ptr, plan->groups,
-                                                  plan->ngroups, plan->window.window,
+                                                  plan->window.ngroups, plan->window.window,
                                                   plan->records, col, (float*)val);
     SB_CHECK_LAUNCH("window_to_csr");
     return SB_OK;

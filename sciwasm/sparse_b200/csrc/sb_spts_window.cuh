@@ -72,6 +72,7 @@ struct Info {
   int window;  // ring slots
   int widest;  // groups of a level at most
   int rows;    // rows of a level at most
+  int ngroups;
 };
 
 // A group: {first row, record offset in 16-byte units, level,
@@ -99,12 +100,13 @@ __host__ __device__ __forceinline__ long long smem_bytes(int window, int tsize) 
 // ------------------------------------------------------------ building
 
 // reach over all rows (natural order): from the first row of the lowest level
-// a row reads to the end of its own level.
+// a row reads to the end of its own level; and the groups of every level
+// (cnt[nlevels + 1], to be scanned).  One thread per row, and one more.
 __global__ void window_reach(const int* __restrict__ row_ptr, const int* __restrict__ col,
                              const int* __restrict__ level, const int* __restrict__ level_ptr,
-                             int N, Info* __restrict__ info) {
+                             int N, int nlevels, int* __restrict__ cnt, Info* __restrict__ info) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int m = 0;
+  int m = 0, rows = 0;
   if (i < N) {
     const int s = row_ptr[i], e = row_ptr[i + 1] - 1;
     int lo = INT_MAX;
@@ -114,29 +116,27 @@ __global__ void window_reach(const int* __restrict__ row_ptr, const int* __restr
     }
     if (lo != INT_MAX) m = level_ptr[level[i] + 1] - level_ptr[lo];
   }
+  if (i < nlevels) rows = level_ptr[i + 1] - level_ptr[i];
+  if (i <= nlevels) cnt[i] = (rows + kGroup - 1) / kGroup;
   m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(&info->reach, m);
-}
-
-// Groups of every level, to be scanned (n = nlevels + 1).
-__global__ void window_level_groups(const int* __restrict__ level_ptr, int nlevels,
-                                    int* __restrict__ cnt, Info* __restrict__ info) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  const int rows = l < nlevels ? level_ptr[l + 1] - level_ptr[l] : 0;
-  if (l <= nlevels) cnt[l] = (rows + kGroup - 1) / kGroup;
-  const int m = __reduce_max_sync(0xffffffffu, rows);
-  if ((threadIdx.x & 31) == 0 && m > 0) {
-    atomicMax(&info->rows, m);
-    atomicMax(&info->widest, (m + kGroup - 1) / kGroup);
+  rows = __reduce_max_sync(0xffffffffu, rows);
+  if ((threadIdx.x & 31) == 0) {
+    if (m > 0) atomicMax(&info->reach, m);
+    if (rows > 0) {
+      atomicMax(&info->rows, rows);
+      atomicMax(&info->widest, (rows + kGroup - 1) / kGroup);
+    }
   }
 }
 
-// Row lengths in level order, and each group's longest row (off-diagonal).
+// Row lengths in level order (N + 1, to be scanned), and each group's longest
+// row (off-diagonal).
 __global__ void window_lengths(const int* __restrict__ row_ptr, const int* __restrict__ perm,
                                const int* __restrict__ level, const int* __restrict__ level_ptr,
                                const int* __restrict__ gstart, int N, int* __restrict__ lens,
                                int4* __restrict__ groups, int* __restrict__ glen) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p == N) lens[N] = 0;
   if (p >= N) return;
   const int src = perm[p];
   const int len = row_ptr[src + 1] - row_ptr[src];
@@ -170,40 +170,47 @@ __host__ __device__ __forceinline__ int unroll_of(int kmax) {
   return kmax <= 3 ? 4 : kmax <= 7 ? 8 : 16;
 }
 
-// Whether to build the layout: it fits (total: the scanned record units, cap:
-// the units there is room for; lower: the structure the solves need), and one
+// Whether to build the layout: it fits (size16: the record units, cap: the
+// units there is room for; lower: the structure the solves need), and one
 // block with its window solves the factor faster than ready flags over the
 // whole GPU.  A block takes a fixed time per group once a level has several,
 // the ready flags a fixed time per level.  Measured on B200 (ns per group at
 // KU 4 / 8 / 16: FP32 24 / 35 / 75, FP64 27 / 51 / 105; us per level of the
 // ready flags: FP32 1.05-1.14, FP64 1.26-1.35), the two meet at about 40, 26
 // and 12 groups per level.
-__global__ void window_decide(const int* __restrict__ total, const int* __restrict__ ngroups,
-                              int nlevels, long long cap, int tsize,
-                              bool lower, Info* __restrict__ info) {
-  const int w = max(kGroup, (info->reach + kGroup - 1) / kGroup * kGroup);
-  const int u = unroll_of(info->kmax);
+__device__ __forceinline__ int window_rows(int reach) {
+  return max(kGroup, (reach + kGroup - 1) / kGroup * kGroup);
+}
+__device__ __forceinline__ bool window_wins(const Info& f, int size16, int ngroups, int nlevels,
+                                            long long cap, int tsize, bool lower) {
+  const int w = window_rows(f.reach), u = unroll_of(f.kmax);
   const int most = u == 4 ? 40 : u == 8 ? 26 : 12;
-  info->size16 = *total;
-  info->window = w;
-  info->use = lower && w <= 0xffff && info->kmax <= kMaxK && *total <= cap &&
-              info->widest <= kMaxArrivals && smem_bytes(w, tsize) <= kSmem &&
-              (long long)*ngroups <= (long long)most * nlevels;
+  return lower && w <= 0xffff && f.kmax <= kMaxK && size16 <= cap && f.widest <= kMaxArrivals &&
+         smem_bytes(w, tsize) <= kSmem && (long long)ngroups <= (long long)most * nlevels;
 }
 
-// Completes the group descriptors and writes the records: one thread per row
-// in level order.
+// Decides, completes the group descriptors and writes the records: one thread
+// per row in level order (gmax: the bound on the number of groups).
 template <typename T>
 __global__ void window_fill(const int* __restrict__ row_ptr, const int* __restrict__ col,
                             const T* __restrict__ val, const int* __restrict__ perm,
                             const int* __restrict__ order, const int* __restrict__ level,
                             const int* __restrict__ level_ptr, const int* __restrict__ gstart,
                             const int* __restrict__ glen, const int* __restrict__ gbase, int N,
-                            const Info* __restrict__ info, int4* __restrict__ groups,
-                            char* __restrict__ records) {
+                            int nlevels, int gmax, long long cap, bool lower, Info* info,
+                            int4* __restrict__ groups, char* __restrict__ records) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= N || !info->use) return;
-  const int w = info->window;
+  if (p >= N) return;
+  const bool use =
+      window_wins(*info, gbase[gmax], gstart[nlevels], nlevels, cap, sizeof(T), lower);
+  const int w = window_rows(info->reach);
+  if (p == 0) {
+    info->size16 = gbase[gmax];
+    info->ngroups = gstart[nlevels];
+    info->window = w;
+    info->use = use;
+  }
+  if (!use) return;
   const int src = perm[p];
   const int l = level[src], i = p - level_ptr[l];
   const int g = gstart[l] + i / kGroup, lane = i % kGroup;
