@@ -6,15 +6,15 @@
 // coo_csr's per-row stable bubble sort makes the result a stable sort of the
 // COO entries by (row, col).  Sorted input (the reference's mmread always
 // quick-sorts by (row, col)) is detected and takes a copy-speed path; other
-// input goes into row buckets whose rows are each sorted by (col, original
-// position) when no row holds more than 2048 entries, and is otherwise
-// ordered by a stable LSD radix sort of packed (row, col) keys whose payload
-// is the original position; either way equal keys keep their COO order.
+// input goes through buckets of rows (sb_buckets.cu) unless a row is too long
+// for them, and is otherwise ordered by a stable LSD radix sort of packed
+// (row, col) keys whose payload is the original position; either way equal keys
+// keep their COO order.
 #include <algorithm>
 
 #include <climits>
 
-#include "sb_common.cuh"
+#include "sb_buckets.cuh"
 #include "sb_prims.cuh"
 
 namespace sb {
@@ -256,403 +256,36 @@ static bool admitted(long long w, long long N, long long nnz) {
   return (wn < 134217728.0) && (ratio <= 5.0);
 }
 
-// ------------------------------------------------------------ coo_csr by row buckets
-// Unsorted COO whose rows hold at most kBucketMaxRow entries: a counting sort
-// by row (an atomic cursor per row hands every entry a slot of its row, in no
-// particular order), then a sort of each row by the key (col << 32 | original
-// position).  The position breaks ties between equal columns, so each row ends
-// up in (col, COO order) -- the stable (row, col) order of the reference's
-// per-row bubble sort -- whatever order the atomics handed out the slots in.
-// One pass over the COO to count, one to scatter 16-byte items, one to sort
-// and store: about 3.5 GB moved for 44M FP64 entries, against the six
-// 8-bit digit passes of the general radix sort.
+constexpr int kCheckPrefix = 1 << 16;
 
-constexpr int kBucketMaxRow = 2048;   // longer rows: the radix sort
-constexpr int kRowThreadMax = 16;     // rows up to this long: one thread, registers
-constexpr int kRowRankMax = 64;       // up to this long: one warp, registers
-constexpr int kRowWarpMax = 256;      // up to this long: one warp, shared memory
-constexpr int kSortWarps = 8;         // warps per block of the warp-per-row kernel
-
-struct BucketItem {
-  unsigned long long key;   // col << 32 | position in the COO
-  unsigned long long bits;  // the value's bits (FP32 in the low half)
-};
-
-__device__ __forceinline__ unsigned long long val_bits(float v) { return __float_as_uint(v); }
-__device__ __forceinline__ unsigned long long val_bits(double v) {
-  return (unsigned long long)__double_as_longlong(v);
-}
-template <typename T> __device__ __forceinline__ T bits_val(unsigned long long b);
-template <> __device__ __forceinline__ float bits_val<float>(unsigned long long b) {
-  return __uint_as_float((unsigned)b);
-}
-template <> __device__ __forceinline__ double bits_val<double>(unsigned long long b) {
-  return __longlong_as_double((long long)b);
-}
-
-__global__ void count_rows(const int* __restrict__ row, long long nnz, int* __restrict__ cnt) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < nnz) atomicAdd(&cnt[row[i]], 1);
-}
-
-__global__ void max_count(const int* __restrict__ cnt, int N, int* __restrict__ out) {
-  int m = 0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < N;
-       i += (long long)gridDim.x * blockDim.x)
-    m = max(m, cnt[i]);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(out, m);
-}
-
-template <typename T>
-__global__ void scatter_rows(const int* __restrict__ row, const int* __restrict__ col,
-                             const T* __restrict__ val, long long nnz, int* __restrict__ cursor,
-                             BucketItem* __restrict__ items) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nnz) return;
-  const int pos = atomicAdd(&cursor[row[i]], 1);
-  BucketItem it;
-  it.key = ((unsigned long long)(unsigned)col[i] << 32) | (unsigned long long)i;
-  it.bits = val_bits(val[i]);
-  items[pos] = it;
-}
-
-template <typename T>
-__device__ __forceinline__ void store_entry(int* col_out, T* val_out, long long p,
-                                            unsigned long long key, unsigned long long bits) {
-  col_out[p] = (int)(key >> 32);
-  val_out[p] = bits_val<T>(bits);
-}
-
-// Bitonic sorting network over registers (n a power of two; indices are
-// compile-time constants after unrolling, so the arrays stay in registers).
-template <int n>
-__device__ __forceinline__ void bitonic_regs(unsigned long long (&k)[n],
-                                             unsigned long long (&b)[n]) {
-#pragma unroll
-  for (int size = 2; size <= n; size <<= 1) {
-#pragma unroll
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-#pragma unroll
-      for (int i = 0; i < n; ++i) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const bool up = (i & size) == 0;
-          const unsigned long long ki = k[i], kj = k[j], bi = b[i], bj = b[j];
-          const bool sw = (ki > kj) == up;
-          k[i] = sw ? kj : ki;
-          k[j] = sw ? ki : kj;
-          b[i] = sw ? bj : bi;
-          b[j] = sw ? bi : bj;
-        }
-      }
-    }
-  }
-}
-
-// One thread per row: rows of up to kRowThreadMax entries are sorted in
-// registers and stored; longer rows are listed for the kernels below, each
-// list read only by the kernel that sorts its rows: up to kRowRankMax entries
-// in lists[0], up to kRowWarpMax in lists[1], longer in lists[2] (counts in
-// n_listed[0..2]).
-template <typename T>
-__global__ void sort_short_rows(const int* __restrict__ row_ptr, int N,
-                                const BucketItem* __restrict__ items, int* __restrict__ col_out,
-                                T* __restrict__ val_out, int* __restrict__ lists, int list_len,
-                                int* __restrict__ n_listed) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= N) return;
-  const int s = row_ptr[r], len = row_ptr[r + 1] - s;
-  if (len == 0) return;
-  if (len > kRowThreadMax) {
-    // one counter add per list and warp (lanes bound for the same list share it)
-    const int which = len <= kRowRankMax ? 0 : (len <= kRowWarpMax ? 1 : 2);
-    const unsigned peers = __match_any_sync(__activemask(), which);
-    const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(n_listed + which, __popc(peers));
-    base = __shfl_sync(peers, base, leader);
-    lists[(long long)which * list_len + base + __popc(peers & ((1u << lane) - 1u))] = r;
-    return;
-  }
-  if (len == 1) {
-    const BucketItem it = items[s];
-    store_entry<T>(col_out, val_out, s, it.key, it.bits);
-    return;
-  }
-  if (len <= 8) {
-    unsigned long long k[8], b[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (j < len) {
-        const BucketItem it = items[s + j];
-        k[j] = it.key;
-        b[j] = it.bits;
-      } else {
-        k[j] = ~0ull;
-        b[j] = 0;
-      }
-    }
-    bitonic_regs<8>(k, b);
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (j < len) store_entry<T>(col_out, val_out, (long long)s + j, k[j], b[j]);
-    return;
-  }
-  unsigned long long k[kRowThreadMax], b[kRowThreadMax];
-#pragma unroll
-  for (int j = 0; j < kRowThreadMax; ++j) {
-    if (j < len) {
-      const BucketItem it = items[s + j];
-      k[j] = it.key;
-      b[j] = it.bits;
-    } else {
-      k[j] = ~0ull;  // above every real key (columns are below 2^31)
-      b[j] = 0;
-    }
-  }
-  bitonic_regs<kRowThreadMax>(k, b);
-#pragma unroll
-  for (int j = 0; j < kRowThreadMax; ++j)
-    if (j < len) store_entry<T>(col_out, val_out, (long long)s + j, k[j], b[j]);
-}
-
-// Bitonic sort of m (a power of two) keys with their bits in shared memory by
-// `nt` cooperating threads numbered t; `sync` orders the steps.  A step's m/2
-// compare-exchange pairs (i, i + stride), i with its stride bit clear, are
-// disjoint; pair p is done by thread p mod nt, so no thread idles in a step.
-struct WarpSync {
-  __device__ __forceinline__ void operator()() const { __syncwarp(); }
-};
-struct BlockSync {
-  __device__ __forceinline__ void operator()() const { __syncthreads(); }
-};
-
-template <typename Sync>
-__device__ __forceinline__ void bitonic_shared(unsigned long long* sk, unsigned long long* sb,
-                                               int m, int t, int nt, Sync sync) {
-  const int half = m >> 1;
-  for (int size = 2; size <= m; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int p = t; p < half; p += nt) {
-        const int i = ((p & ~(stride - 1)) << 1) | (p & (stride - 1));
-        const int j = i + stride;
-        const bool up = (i & size) == 0;
-        const unsigned long long ki = sk[i], kj = sk[j];
-        if ((ki > kj) == up) {
-          sk[i] = kj;
-          sk[j] = ki;
-          const unsigned long long bi = sb[i];
-          sb[i] = sb[j];
-          sb[j] = bi;
-        }
-      }
-      sync();
-    }
-  }
-}
-
-// One warp per row of kRowThreadMax+1 .. kRowRankMax entries: each lane holds
-// entries lane and lane + 32 in registers and counts, over all the row's keys
-// broadcast by shuffles, how many are smaller; that count is the entry's slot
-// (keys are distinct: they hold the position).  No shared memory, so every
-// warp slot of an SM can hold a row in flight.
-template <typename T>
-__global__ void __launch_bounds__(256)
-    sort_rank_rows(const int* __restrict__ row_ptr, const BucketItem* __restrict__ items,
-                   const int* __restrict__ rows, const int* __restrict__ n_rows,
-                   int* __restrict__ col_out, T* __restrict__ val_out) {
-  const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-  const int n = *n_rows;
-  for (int q = blockIdx.x * wpb + (threadIdx.x >> 5); q < n; q += gridDim.x * wpb) {
-    const int r = rows[q];
-    const int s = row_ptr[r], len = row_ptr[r + 1] - s;
-    unsigned long long k0 = ~0ull, b0 = 0, k1 = ~0ull, b1 = 0;
-    if (lane < len) {
-      const BucketItem it = items[s + lane];
-      k0 = it.key;
-      b0 = it.bits;
-    }
-    if (lane + 32 < len) {
-      const BucketItem it = items[s + 32 + lane];
-      k1 = it.key;
-      b1 = it.bits;
-    }
-    int r0 = 0, r1 = 0;
-    if (len <= 32) {
-      for (int j = 0; j < len; ++j) r0 += __shfl_sync(0xffffffffu, k0, j) < k0;
-    } else {
-#pragma unroll 4
-      for (int j = 0; j < 32; ++j) {
-        const unsigned long long a = __shfl_sync(0xffffffffu, k0, j);
-        const unsigned long long c = __shfl_sync(0xffffffffu, k1, j);
-        r0 += (a < k0) + (c < k0);
-        r1 += (a < k1) + (c < k1);
-      }
-    }
-    if (lane < len) store_entry<T>(col_out, val_out, (long long)s + r0, k0, b0);
-    if (lane + 32 < len) store_entry<T>(col_out, val_out, (long long)s + r1, k1, b1);
-  }
-}
-
-// One warp per row of kRowRankMax+1 .. kRowWarpMax entries: a bitonic sort in
-// the warp's shared memory.
-template <typename T>
-__global__ void __launch_bounds__(kSortWarps * 32)
-    sort_warp_rows(const int* __restrict__ row_ptr, const BucketItem* __restrict__ items,
-                   const int* __restrict__ rows, const int* __restrict__ n_rows,
-                   int* __restrict__ col_out, T* __restrict__ val_out) {
-  __shared__ unsigned long long sk[kSortWarps][kRowWarpMax];
-  __shared__ unsigned long long sb[kSortWarps][kRowWarpMax];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = *n_rows;
-  for (int q = blockIdx.x * kSortWarps + warp; q < n; q += gridDim.x * kSortWarps) {
-    const int r = rows[q];
-    const int s = row_ptr[r], len = row_ptr[r + 1] - s;
-    int m = 128;
-    while (m < len) m <<= 1;
-    for (int t = lane; t < m; t += 32) {
-      if (t < len) {
-        const BucketItem it = items[s + t];
-        sk[warp][t] = it.key;
-        sb[warp][t] = it.bits;
-      } else {
-        sk[warp][t] = ~0ull;
-        sb[warp][t] = 0;
-      }
-    }
-    __syncwarp();
-    bitonic_shared(sk[warp], sb[warp], m, lane, 32, WarpSync());
-    for (int t = lane; t < len; t += 32)
-      store_entry<T>(col_out, val_out, (long long)s + t, sk[warp][t], sb[warp][t]);
-    __syncwarp();
-  }
-}
-
-// One block per listed row of kRowWarpMax+1 .. kBucketMaxRow entries.
-constexpr int kBlockSortThreads = 512;
-
-template <typename T>
-__global__ void __launch_bounds__(kBlockSortThreads)
-    sort_block_rows(const int* __restrict__ row_ptr, const BucketItem* __restrict__ items,
-                    const int* __restrict__ long_rows, const int* __restrict__ n_long,
-                    int* __restrict__ col_out, T* __restrict__ val_out) {
-  __shared__ unsigned long long sk[kBucketMaxRow];
-  __shared__ unsigned long long sb[kBucketMaxRow];
-  const int n = *n_long;
-  for (int q = blockIdx.x; q < n; q += gridDim.x) {
-    const int r = long_rows[q];
-    const int s = row_ptr[r], len = row_ptr[r + 1] - s;
-    int m = 512;
-    while (m < len) m <<= 1;
-    for (int t = threadIdx.x; t < m; t += blockDim.x) {
-      if (t < len) {
-        const BucketItem it = items[s + t];
-        sk[t] = it.key;
-        sb[t] = it.bits;
-      } else {
-        sk[t] = ~0ull;
-        sb[t] = 0;
-      }
-    }
-    __syncthreads();
-    bitonic_shared(sk, sb, m, threadIdx.x, blockDim.x, BlockSync());
-    for (int t = threadIdx.x; t < len; t += blockDim.x)
-      store_entry<T>(col_out, val_out, (long long)s + t, sk[t], sb[t]);
-    __syncthreads();
-  }
-}
-
-static int device_sm_count() {
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
-    return 148;
-  return n;
-}
-
-// Returns SB_OK, an error, or kBucketFallBack when a row is longer than
-// kBucketMaxRow (nothing has been written then).
-constexpr int kBucketFallBack = 1;
-
-template <typename T>
-static int coo_csr_buckets(const int* row, const int* col, const T* val, int N, long long nnz,
-                           int* csr_row, int* csr_col, T* csr_val, cudaStream_t st) {
-  // cnt[N + 1], lists[3][N] (rows for the rank, warp and block sorts),
-  // misc[4] = {max row, rows listed for each of the three sorts}
-  int* small = nullptr;
-  const size_t small_ints = 4 * (size_t)N + 5;
-  int r = scratch_alloc((void**)&small, sizeof(int) * small_ints, st);
+// coo_check's flags for the first n entries, on the host.
+static int check_order(const int* row, const int* col, long long n, int N, int (&hf)[2],
+                       cudaStream_t st) {
+  int* flags = nullptr;
+  const int r = scratch_alloc((void**)&flags, 2 * sizeof(int), st);
   if (r) return r;
-  int* cnt = small;
-  int* lists = small + N + 1;
-  int* misc = small + 4 * (size_t)N + 1;
-  BucketItem* items = nullptr;
-  const int sms = device_sm_count();
-  cudaError_t e = cudaMemsetAsync(small, 0, sizeof(int) * small_ints, st);
-  if (e == cudaSuccess) {
-    count_rows<<<grid_for(nnz), kThreads, 0, st>>>(row, nnz, cnt);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) {
-    max_count<<<std::min<unsigned>(grid_for(N), 4u * sms), kThreads, 0, st>>>(cnt, N, misc);
-    e = cudaGetLastError();
-  }
-  int maxlen = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&maxlen, misc, sizeof(int), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) r = cuda_status(e, "coo_csr (row counts)");
-  if (!r && maxlen > kBucketMaxRow) r = kBucketFallBack;
-  if (!r) r = prim::exclusive_scan(cnt, csr_row, (long long)N + 1, st);  // cnt[N] = 0
-  if (!r) r = scratch_alloc((void**)&items, sizeof(BucketItem) * (size_t)nnz, st);
-  if (!r) {
-    e = cudaMemcpyAsync(cnt, csr_row, sizeof(int) * (size_t)N, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) {
-      scatter_rows<T><<<grid_for(nnz), kThreads, 0, st>>>(row, col, val, nnz, cnt, items);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) {
-      sort_short_rows<T><<<grid_for(N), kThreads, 0, st>>>(csr_row, N, items, csr_col, csr_val,
-                                                           lists, N, misc + 1);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess && maxlen > kRowThreadMax) {
-      sort_rank_rows<T><<<8 * sms, 256, 0, st>>>(csr_row, items, lists, misc + 1, csr_col,
-                                                 csr_val);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess && maxlen > kRowRankMax) {
-      sort_warp_rows<T><<<4 * sms, kSortWarps * 32, 0, st>>>(csr_row, items, lists + N, misc + 2,
-                                                             csr_col, csr_val);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess && maxlen > kRowWarpMax) {
-      sort_block_rows<T><<<4 * sms, kBlockSortThreads, 0, st>>>(
-          csr_row, items, lists + 2 * (size_t)N, misc + 3, csr_col, csr_val);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) r = cuda_status(e, "coo_csr (row buckets)");
-  }
-  if (items) scratch_free(items, st);
-  scratch_free(small, st);
-  return r;
+  SB_CHECK_CUDA(cudaMemsetAsync(flags, 0, 2 * sizeof(int), st));
+  coo_check<<<grid_for(n, kThreads * kCheckItems), kThreads, 0, st>>>(row, col, n, N, flags);
+  SB_CHECK_LAUNCH("coo_check");
+  SB_CHECK_CUDA(cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, st));
+  SB_CHECK_CUDA(cudaStreamSynchronize(st));
+  scratch_free(flags, st);
+  return SB_OK;
 }
 
 template <typename T>
 static int coo_csr_impl(const int* row, const int* col, const T* val, int N, long long nnz,
                         int* csr_row, int* csr_col, T* csr_val, cudaStream_t st) {
-  int* flags = nullptr;
-  int r = scratch_alloc((void**)&flags, 2 * sizeof(int), st);
-  if (r) return r;
-  SB_CHECK_CUDA(cudaMemsetAsync(flags, 0, 2 * sizeof(int), st));
-  coo_check<<<grid_for(nnz, kThreads * kCheckItems), kThreads, 0, st>>>(row, col, nnz, N, flags);
-  SB_CHECK_LAUNCH("coo_check");
+  // the order of a prefix first: shuffled entries show there, and then their
+  // indices are checked by the pass that counts them
   int hf[2] = {0, 0};
-  SB_CHECK_CUDA(cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, st));
-  SB_CHECK_CUDA(cudaStreamSynchronize(st));
-  scratch_free(flags, st);
+  long long checked = std::min(nnz, (long long)kCheckPrefix);
+  int r = check_order(row, col, checked, N, hf, st);
+  if (!r && !hf[0] && !hf[1] && checked < nnz) {
+    checked = nnz;
+    r = check_order(row, col, nnz, N, hf, st);
+  }
+  if (r) return r;
   if (hf[0]) {
     set_error("coo_csr: row or column index outside [0, N)");
     return SB_EINVAL;
@@ -665,10 +298,11 @@ static int coo_csr_impl(const int* row, const int* col, const T* val, int N, lon
     SB_CHECK_LAUNCH("row_ptr_from_sorted");
     return SB_OK;
   }
-  // general order, rows of at most kBucketMaxRow entries: row buckets
-  r = coo_csr_buckets<T>(row, col, val, N, nnz, csr_row, csr_col, csr_val, st);
-  if (r != kBucketFallBack) return r;
-  // longer rows: stable radix sort of (row << 32 | col) with positions
+  // any order: buckets of rows
+  r = bucket_csr<T>(row, col, nullptr, val, N, N, nnz, checked < nnz, csr_row, csr_col,
+                    csr_val, st);
+  if (r != kBucketsUnfit) return r;
+  // rows beyond a bucket: stable radix sort of (row << 32 | col) with positions
   prim::RadixBuffers b;
   void* mem = nullptr;
   const size_t kb = sizeof(unsigned long long) * (size_t)nnz, vb = sizeof(unsigned) * (size_t)nnz;

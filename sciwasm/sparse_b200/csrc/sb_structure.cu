@@ -12,7 +12,7 @@
 // radix sort with the original position as payload.
 #include <algorithm>
 
-#include "sb_common.cuh"
+#include "sb_buckets.cuh"
 #include "sb_prims.cuh"
 
 namespace sb {
@@ -155,7 +155,8 @@ __global__ void ell_copy_nz(const T* __restrict__ data, const int* __restrict__ 
   }
 }
 
-// transpose_csr: sort entries (storage order) stably by column.
+// transpose_csr with a column too long for a bucket: sort entries (storage
+// order) stably by column.
 __global__ void col_keys(const int* __restrict__ col, long long nnz,
                          unsigned long long* __restrict__ k, unsigned* __restrict__ v) {
   const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -336,10 +337,13 @@ static int transpose_csr_impl(const int* row_ptr, const int* col, const T* val, 
     SB_CHECK_CUDA(cudaStreamSynchronize(st));
     return SB_OK;
   }
+  int r = bucket_csr<T>(col, nullptr, row_ptr, val, N, N, nnz, true, orow_ptr, ocol, oval, st);
+  if (r != kBucketsUnfit) return r;
+  // a column beyond a bucket: a stable radix sort by column
   prim::RadixBuffers b;
   void* mem = nullptr;
   const size_t kb = sizeof(unsigned long long) * nnz, vb = sizeof(unsigned) * nnz;
-  int r = scratch_alloc(&mem, 2 * kb + 2 * vb + 2 * sizeof(int) * nnz, st);
+  r = scratch_alloc(&mem, 2 * kb + 2 * vb + 2 * sizeof(int) * nnz, st);
   if (r) return r;
   char* p = (char*)mem;
   b.k[0] = (unsigned long long*)p;
