@@ -54,6 +54,11 @@ const char* sb_last_error(void);
 const char* sb_status_string(int status);
 int sb_device_count(int* count);
 int sb_set_device(int device);
+/* Device memory of the current device.  sb_free may be called while work that
+ * uses the block is in flight and does not wait for it: freed blocks are kept
+ * (up to 2 GiB per device) and handed out again only after a device
+ * synchronisation; they go back to the driver when an allocation fails, and
+ * sb_mem_info counts them as free. */
 int sb_malloc(void** ptr, size_t bytes);
 int sb_free(void* ptr);
 int sb_host_alloc(void** ptr, size_t bytes); /* pinned host memory */

@@ -706,9 +706,9 @@ static void exec_release(sb_batch_exec* e) {
     if (b.h_items) cudaFreeHost(b.h_items);
     if (b.h_offsets) cudaFreeHost(b.h_offsets);
     if (b.h_count) cudaFreeHost(b.h_count);
-    if (b.d_items) cudaFree(b.d_items);
-    if (b.d_offsets) cudaFree(b.d_offsets);
-    if (b.d_count) cudaFree(b.d_count);
+    device_free(b.d_items);
+    device_free(b.d_offsets);
+    device_free(b.d_count);
   }
   if (e->capture_stream) cudaStreamDestroy(e->capture_stream);
   delete e;
@@ -830,9 +830,12 @@ int sb_batch_exec_create(int dtype, int32_t capacity, sb_batch_exec** out) {
     SB_E(cudaMallocHost(&b.h_items, sizeof(sb_batch_item) * capacity));
     SB_E(cudaMallocHost(&b.h_offsets, sizeof(long long) * (capacity + 1)));
     SB_E(cudaMallocHost(&b.h_count, sizeof(int) * 4));
-    SB_E(cudaMalloc(&b.d_items, sizeof(sb_batch_item) * capacity));
-    SB_E(cudaMalloc(&b.d_offsets, sizeof(long long) * (capacity + 1)));
-    SB_E(cudaMalloc(&b.d_count, sizeof(int) * 4));
+    if ((r = device_alloc((void**)&b.d_items, sizeof(sb_batch_item) * capacity)) ||
+        (r = device_alloc((void**)&b.d_offsets, sizeof(long long) * (capacity + 1))) ||
+        (r = device_alloc((void**)&b.d_count, sizeof(int) * 4))) {
+      exec_release(e);
+      return r;
+    }
     SB_E(cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming));
     // capture: descriptors + offsets + item count (host -> device, the
     // count's copy also resets the work counter), persistent kernel

@@ -57,6 +57,11 @@ int sm_count();
 // timeout; read and cleared by sb_device_status().
 int* device_status_word();
 
+// Device memory of objects that outlive a call (sb_malloc and sb_free): freed
+// blocks are kept for reuse within a bound.
+int device_alloc(void** p, size_t bytes);
+int device_free(void* p);
+
 // Scratch allocation ordered on a stream (stream-ordered pool).
 int scratch_alloc(void** p, size_t bytes, cudaStream_t s);
 void scratch_free(void* p, cudaStream_t s);

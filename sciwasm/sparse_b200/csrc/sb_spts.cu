@@ -1032,13 +1032,13 @@ static int polling_grid(const void* kern, int algo, int N, int nlevels) {
   return std::min(full, sm_count());
 }
 
-// The plan's device arrays live in one allocation (one cudaMalloc per plan,
+// The plan's device arrays live in one allocation (one per plan,
 // not one per array); level_ptr is sized for the largest possible level
 // count, N + 1 (a row's level is at most its index + 1).
 static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 static void plan_release(sb_spts_plan* p) {
-  for (void* q : p->owned) cudaFree(q);
+  for (void* q : p->owned) device_free(q);
   p->owned.clear();
   if (p->ev[0]) cudaEventDestroy(p->ev[0]);
   if (p->ev[1]) cudaEventDestroy(p->ev[1]);
@@ -1079,8 +1079,7 @@ static int analyze_impl(sb_spts_plan* p, cudaStream_t st) {
     size_t total = 0;
     for (size_t b : sizes) total += align256(b);
     void* slab = nullptr;
-    cudaError_t e = cudaMalloc(&slab, total);
-    if (e != cudaSuccess) return cuda_status(e, "sb_spts_analyze: cudaMalloc");
+    if ((r = device_alloc(&slab, total))) return r;
     p->owned.push_back(slab);
     char* q = (char*)slab;
     void* part[9];
@@ -1387,7 +1386,7 @@ static void spts_batch_release(sb_spts_batch* e) {
   if (e->graph_def) cudaGraphDestroy(e->graph_def);
   if (e->done) cudaEventDestroy(e->done);
   if (e->h) cudaFreeHost(e->h);
-  if (e->d) cudaFree(e->d);
+  device_free(e->d);
   delete e;
 }
 
@@ -1598,7 +1597,10 @@ int sb_spts_batch_create(int dtype, int policy, int32_t capacity, sb_spts_batch*
   e->moves = part(msize * cap);
   e->count = part(sizeof(int));
   SB_E(cudaMallocHost(&e->h, e->bytes));
-  SB_E(cudaMalloc(&e->d, e->bytes));
+  if ((r = device_alloc((void**)&e->d, e->bytes))) {
+    spts_batch_release(e);
+    return r;
+  }
   SB_E(cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming));
   memset(e->h, 0, e->bytes);
   e->limit = kDefaultSpin;

@@ -1,0 +1,105 @@
+"""Device memory that is kept after sb_free: reuse waits for work in flight on
+other streams, blocks are handed out once, double frees are refused, the bound
+holds, a failing allocation gives the kept blocks back, and threads may allocate
+and free at the same time."""
+import ctypes
+import threading
+
+import numpy as np
+import pytest
+
+from sciwasm.sparse_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+MIB = 1 << 20
+
+
+def _alloc(n):
+    p = ctypes.c_void_p()
+    _lib.call("sb_malloc", ctypes.byref(p), n)
+    return p.value
+
+
+def _info():
+    free, total = ctypes.c_size_t(), ctypes.c_size_t()
+    _lib.call("sb_mem_info", ctypes.byref(free), ctypes.byref(total))
+    return free.value, total.value
+
+
+def test_reuse_waits_for_the_old_use(gpu):
+    """A long chain of copies out of a block on one stream; the block is freed
+    and allocated again meanwhile, and overwritten on another stream."""
+    n = 256 * MIB
+    streams = []
+    for _ in range(2):
+        s = ctypes.c_void_p()
+        _lib.call("sb_stream_create", ctypes.byref(s))
+        streams.append(s.value)
+    src, dst = _alloc(n), _alloc(n)
+    _lib.call("sb_memset", src, 0x5A, n, streams[0])
+    for _ in range(40):
+        _lib.call("sb_memcpy_dtod", dst, src, n, streams[0])
+    _lib.call("sb_free", src)
+    again = _alloc(n)
+    _lib.call("sb_memset", again, 0, n, streams[1])
+    _lib.call("sb_stream_synchronize", streams[0])
+    _lib.call("sb_stream_synchronize", streams[1])
+    out = np.empty(n, np.uint8)
+    _lib.call("sb_memcpy_dtoh", out.ctypes.data, dst, n, None)
+    _lib.call("sb_stream_synchronize", None)
+    assert again == src and np.all(out == 0x5A)
+    for p in (again, dst):
+        _lib.call("sb_free", p)
+    for s in streams:
+        _lib.call("sb_stream_destroy", s)
+
+
+def test_double_free_and_distinct_blocks(gpu):
+    lib = _lib.load()
+    ps = [_alloc(3 * MIB) for _ in range(4)]
+    assert len(set(ps)) == 4
+    for p in ps:
+        assert lib.sb_free(p) == 0
+    assert lib.sb_free(ps[0]) < 0
+    qs = [_alloc(3 * MIB) for _ in range(4)]
+    assert len(set(qs)) == 4
+    for q in qs:
+        assert lib.sb_free(q) == 0
+
+
+def test_bound_and_giving_back(gpu):
+    free0, total = _info()
+    ps = [_alloc(512 * MIB) for _ in range(8)]
+    for p in ps:
+        _lib.call("sb_free", p)
+    free1, _ = _info()
+    assert free1 >= free0 - 64 * MIB  # kept blocks count as free
+    big = free1 - 1024 * MIB          # does not fit beside 2 GiB of kept blocks
+    p = _alloc(big)
+    _lib.call("sb_free", p)
+    lib = _lib.load()
+    q = ctypes.c_void_p()
+    assert lib.sb_malloc(ctypes.byref(q), total * 2) == _lib.SB_ENOMEM and not q.value
+    assert lib.sb_malloc(ctypes.byref(q), MIB) == 0
+    _lib.call("sb_free", q.value)
+
+
+def test_threads(gpu):
+    bad = []
+
+    def work(seed):
+        rng = np.random.default_rng(seed)
+        for _ in range(40):
+            a = gpu.DeviceArray.from_host(np.full(int(rng.integers(1, 200_000)), seed, np.int32))
+            b = gpu.DeviceArray.from_host(np.full(1000, -seed, np.int32))
+            if not (np.all(a.to_host() == seed) and np.all(b.to_host() == -seed)):
+                bad.append(seed)
+            a.free()
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(1, 7)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
