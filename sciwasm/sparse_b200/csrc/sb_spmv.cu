@@ -363,7 +363,13 @@ __global__ void __launch_bounds__(256, Out::template min_blocks<T>())
                     const SV* __restrict__ val, const T* __restrict__ x, const T* y_in,
                     Out out, int N) {
   constexpr int RPB = kWarp / V;           // rows per batch
-  constexpr int SHORT = V * UNROLL;        // a short row needs one unrolled pass
+  constexpr int PASS = V * UNROLL;         // entries of one unrolled pass
+  // A short row needs one pass, or two where a second pass measured faster than
+  // the whole-warp tail (power-law 2M FP64, V = 8: 248 -> 232 us, V = 4: 270 ->
+  // 238; but V = 8 with f32 sums 201 -> 211, V = 2 on the banded 4M FP64 matrix
+  // 124 -> 129, V = 1 on the 4096^2 Laplacian 166 -> 176)
+  constexpr int PASSES = (V == 4 || (V == 8 && sizeof(T) == 8)) ? 2 : 1;
+  constexpr int SHORT = PASSES * PASS;
   constexpr bool COMP = sizeof(T) == 4;    // compensate long f32 sums
   const int lane = threadIdx.x & (kWarp - 1);
   const int g = lane / V;
@@ -384,20 +390,26 @@ __global__ void __launch_bounds__(256, Out::template min_blocks<T>())
       const int e = __shfl_sync(kFull, e_l, j);
       const int len = e - s;
       T sum = 0;
-      if (len <= SHORT) {
+      auto pass = [&](int k0) {
         int cc[UNROLL];
         T vv[UNROLL];
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u) {
-          const int k = s + q + u * V;
+          const int k = k0 + u * V;
           cc[u] = k < e ? ld_reuse(col + k) : 0;
           vv[u] = k < e ? (T)ld_val_reuse(val + k) : (T)0;
         }
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u) {
-          const int k = s + q + u * V;
+          const int k = k0 + u * V;
           if (k < e) sum += vv[u] * ld_ro(x + cc[u]);
         }
+      };
+      if constexpr (PASSES == 1) {
+        if (len <= SHORT) pass(s + q);
+      } else {
+        for (int k0 = s + q; __any_sync(kFull, k0 < e && len <= SHORT); k0 += PASS)
+          if (len <= SHORT) pass(k0);
       }
 #pragma unroll
       for (int off = V >> 1; off > 0; off >>= 1) sum += __shfl_xor_sync(kFull, sum, off);
@@ -476,13 +488,30 @@ static int launch_csr_rows_u(const int* row_ptr, const int* col, const SV* val, 
   return launch_csr_rows_v<SV, T, V, 4>(row_ptr, col, val, x, y_in, out, N, grid, st);
 }
 
-// Default lanes per row from the mean row length (about three items per lane).
+// Lanes per row from the mean row length (about three items per lane): the
+// middle of the autotuner's candidates.
 static int default_lanes(int N, long long nnz) {
   const double avg = N ? (double)nnz / N : 0.0;
   if (avg <= 6) return 2;
   if (avg <= 14) return 4;
   if (avg <= 28) return 8;
   return 16;
+}
+
+// Options of a call that gives none, from the mean row length.  Few lanes with
+// a long unroll for short rows: a lane's loads of consecutive entries share
+// sectors, and no shuffle follows.  One warp per block of rows for longer ones,
+// whose lengths usually differ.  Measured on B200 (us, with the lanes above,
+// unroll 4 and the resident grid -> now): Laplacian 4096^2 FP32 199 -> 166, FP64
+// 252 -> 234; banded 4M x 11 FP64 125 -> 119, FP32 98 -> 86; power-law 2M FP64
+// 256 -> 232, FP32 225 -> 199; rows of Poisson(5) entries, random columns, 1M
+// rows FP32 43 -> 41, FP64 43 -> 45.
+static sb_csr_opts default_opts(int N, long long nnz) {
+  const double avg = N ? (double)nnz / N : 0.0;
+  if (avg <= 6) return {0, 1, 8, 0};
+  if (avg <= 14) return {0, 2, 8, 0};
+  if (avg <= 28) return {0, 8, 4, 1};
+  return {0, 16, 4, 1};
 }
 
 template <typename SV, typename T, class Out>
@@ -1487,8 +1516,9 @@ static int launch_csr(const int* row_ptr, const int* col, const S* val, const S*
     if (opts->unroll == 2048) return launch_csr_stream<S, 2048, 3>(row_ptr, col, val, x, y, N, nnz, st);
     return launch_csr_stream<S, 1024, 4>(row_ptr, col, val, x, y, N, nnz, st);
   }
-  return launch_csr_rows<S, S>(row_ptr, col, val, x, y, N, nnz, opts ? opts->lanes_per_row : 0,
-                               opts ? opts->unroll : 0, opts ? opts->grid : 0, st);
+  const sb_csr_opts o = opts ? *opts : default_opts(N, nnz);
+  return launch_csr_rows<S, S>(row_ptr, col, val, x, y, N, nnz, o.lanes_per_row, o.unroll, o.grid,
+                               st);
 }
 
 template <typename S, typename A>
@@ -1548,8 +1578,8 @@ int sb_spmv_csr_allgather(int dtype, const int32_t* row_ptr, const int32_t* col,
   int r = ensure_device();
   if (r) return r;
   cudaStream_t st = as_stream(stream);
-  const int lanes = opts ? opts->lanes_per_row : 0, unroll = opts ? opts->unroll : 0;
-  const int grid = opts ? opts->grid : 0;
+  const sb_csr_opts o = opts ? *opts : default_opts(rows, nnz);
+  const int lanes = o.lanes_per_row, unroll = o.unroll, grid = o.grid;
   const unsigned long long* dd = reinterpret_cast<const unsigned long long*>(dst);
   if (dtype == SB_F64) {
     YScatter<double> out{};
@@ -1601,12 +1631,12 @@ int sb_spmv_csr_ex(int dtype, const int32_t* row_ptr, const int32_t* col, const 
     else if (dtype == SB_BF16 && opts && opts->kernel == 3)
       r = launch_csr_block_stream<__nv_bfloat16, float>(row_ptr, col, (const __nv_bfloat16*)val,
                                                         (const float*)x, (float*)y, N, nnz, st);
-    else if (dtype == SB_BF16)
+    else if (dtype == SB_BF16) {
+      const sb_csr_opts o = opts ? *opts : default_opts(N, nnz);
       r = launch_csr_rows<__nv_bfloat16, float>(row_ptr, col, (const __nv_bfloat16*)val,
                                                 (const float*)x, (float*)y, N, nnz,
-                                                opts ? opts->lanes_per_row : 0,
-                                                opts ? opts->unroll : 0, opts ? opts->grid : 0,
-                                                st);
+                                                o.lanes_per_row, o.unroll, o.grid, st);
+    }
     else if (dtype == SB_F32)
       r = launch_csr<float, float>(row_ptr, col, (const float*)val, (const float*)x, (float*)y, N,
                                    nnz, opts, st);
