@@ -411,6 +411,7 @@ int bucket_csr(const int* row, const int* col, const int* csr_ptr, const T* val,
         e = cudaGetLastError();
       }
     }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) r = cuda_status(e, "bucket_csr");
   }
   if (items) scratch_free(items, st);
