@@ -7,7 +7,7 @@
 //   transpose_ell :6634; COO transpose swaps the index arrays
 //   (src/sequential/src/sparse32.js:1106-1115).
 // The nonzero test everywhere is v > 0 || v < 0 (+0, -0 and NaN are zeros).
-// Ordered compactions use an exclusive scan of the keep flags; orderings
+// Ordered compactions use an exclusive scan of the kept counts; orderings
 // that the reference gets from sequential counting sorts use the stable
 // radix sort with the original position as payload.
 #include <algorithm>
@@ -36,29 +36,90 @@ __global__ void count_nz(const T* __restrict__ v, long long n, unsigned long lon
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
 }
 
-template <typename T>
-__global__ void nz_flags(const T* __restrict__ v, long long n, int* __restrict__ f) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) f[i] = nz(v[i]) ? 1 : 0;
-  else if (i == n) f[i] = 0;
-}
+// Ordered compaction of the nonzero entries in two passes over the values: a
+// count per tile, and (tile counts scanned) the copy, in which a warp walks
+// its 32-entry words, a ballot giving each kept entry its place.  With row
+// pointers to translate, every word's kept bits and first place are kept (8
+// bytes per 32 entries) so that a row's start is a lookup.  One flag and one
+// place per entry, scanned, took 0.29 ms for 20M FP32 entries on B200
+// (flags 58 us, scan 115, copy 113, pointers 16); now 0.10 (the copy 49).
+constexpr int kTileWords = 8;                          // words of a warp
+constexpr int kTileEntries = kTh * kTileWords;         // entries of a block: 2048
 
 template <typename T>
-__global__ void scatter_nz_coo(const int* __restrict__ row, const int* __restrict__ col,
-                               const T* __restrict__ val, long long n, const int* __restrict__ pos,
-                               int* __restrict__ orow, int* __restrict__ ocol, T* __restrict__ oval) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !nz(val[i])) return;
-  const int p = pos[i];
-  if (orow) orow[p] = row[i];
-  ocol[p] = col[i];
-  oval[p] = val[i];
+__global__ void __launch_bounds__(kTh)
+    nz_tiles(const T* __restrict__ v, long long n, int* __restrict__ sums) {
+  __shared__ int total;
+  if (threadIdx.x == 0) total = 0;
+  const long long base = (long long)blockIdx.x * kTileEntries + threadIdx.x;
+  int c = 0;
+#pragma unroll
+  for (int u = 0; u < kTileWords; ++u) {
+    const long long i = base + u * kTh;
+    c += i < n && nz(v[i]);
+  }
+  c = __reduce_add_sync(0xffffffffu, c);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) atomicAdd(&total, c);
+  __syncthreads();
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-__global__ void rowptr_through(const int* __restrict__ row_ptr, int N, const int* __restrict__ pos,
-                               int* __restrict__ orow_ptr) {
+// words: {kept bits, place of the word's first kept entry} or null.
+template <typename T>
+__global__ void __launch_bounds__(kTh)
+    nz_compact(const int* __restrict__ row, const int* __restrict__ col,
+               const T* __restrict__ val, long long n, const int* __restrict__ tile_start,
+               uint2* __restrict__ words, int* __restrict__ orow, int* __restrict__ ocol,
+               T* __restrict__ oval) {
+  __shared__ int warp_sum[kTh / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long first = (long long)blockIdx.x * kTileEntries + warp * (32 * kTileWords);
+  T v[kTileWords];
+  unsigned bits[kTileWords];
+  int total = 0;
+#pragma unroll
+  for (int u = 0; u < kTileWords; ++u) {
+    const long long i = first + u * 32 + lane;
+    v[u] = i < n ? val[i] : T(0);
+  }
+#pragma unroll
+  for (int u = 0; u < kTileWords; ++u) {
+    bits[u] = __ballot_sync(0xffffffffu, nz(v[u]));  // (entries past n are zeros)
+    total += __popc(bits[u]);
+  }
+  if (lane == 0) warp_sum[warp] = total;
+  __syncthreads();
+  int at = tile_start[blockIdx.x];
+  for (int w = 0; w < warp; ++w) at += warp_sum[w];
+#pragma unroll
+  for (int u = 0; u < kTileWords; ++u) {
+    const long long i = first + u * 32 + lane;
+    if (words && lane == 0 && first + u * 32 < n)
+      words[(first >> 5) + u] = make_uint2(bits[u], (unsigned)at);
+    if (bits[u] & (1u << lane)) {
+      const int p = at + __popc(bits[u] & ((1u << lane) - 1u));
+      if (orow) orow[p] = row[i];
+      ocol[p] = col[i];
+      oval[p] = v[u];
+    }
+    at += __popc(bits[u]);
+  }
+}
+
+// Row pointers through the compaction (total: kept entries).
+__global__ void nz_row_ptr(const int* __restrict__ row_ptr, int N, long long n,
+                           const uint2* __restrict__ words, const int* __restrict__ total,
+                           int* __restrict__ orow_ptr) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i <= N) orow_ptr[i] = pos[row_ptr[i]];
+  if (i > N) return;
+  const int j = row_ptr[i];
+  if (j >= n) {
+    orow_ptr[i] = *total;
+    return;
+  }
+  const uint2 w = words[j >> 5];
+  orow_ptr[i] = (int)w.y + __popc(w.x & ((1u << (j & 31)) - 1u));
 }
 
 // DIA: keep flags over the virtual (diagonal, row) grid d*N + n, in-band only.
@@ -265,22 +326,37 @@ static int count_nz_impl(const T* v, long long n, long long* count, cudaStream_t
 template <typename T>
 static int copy_nz_impl(const int* row_ptr, int N, const int* row, const int* col, const T* val,
                         long long n, int* orow_or_ptr, int* ocol, T* oval, cudaStream_t st) {
-  int* pos = nullptr;
-  int r = scratch_alloc((void**)&pos, sizeof(int) * (size_t)(n + 1), st);
+  if (n == 0) {  // (a CSR without entries)
+    SB_CHECK_CUDA(cudaMemsetAsync(orow_or_ptr, 0, sizeof(int) * ((size_t)N + 1), st));
+    SB_CHECK_CUDA(cudaStreamSynchronize(st));
+    return SB_OK;
+  }
+  // words (8 bytes per 32 entries, for row pointers), tile starts and the total
+  const long long tiles = (n + kTileEntries - 1) / kTileEntries;
+  const size_t wbytes = row_ptr ? sizeof(uint2) * (size_t)((n + 31) / 32) : 0;
+  char* mem = nullptr;
+  int r = scratch_alloc((void**)&mem, wbytes + sizeof(int) * (size_t)(tiles + 1), st);
   if (r) return r;
-  nz_flags<T><<<g1(n + 1), kTh, 0, st>>>(val, n, pos);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) r = cuda_status(e, "nz_flags");
-  if (!r) r = prim::exclusive_scan(pos, pos, n + 1, st);
-  if (!r) {
-    scatter_nz_coo<T><<<g1(n), kTh, 0, st>>>(row, col, val, n, pos, row_ptr ? nullptr : orow_or_ptr,
-                                              ocol, oval);
-    if (row_ptr) rowptr_through<<<g1((long long)N + 1), kTh, 0, st>>>(row_ptr, N, pos, orow_or_ptr);
+  uint2* words = row_ptr ? (uint2*)mem : nullptr;
+  int* start = (int*)(mem + wbytes);
+  cudaError_t e = cudaMemsetAsync(start + tiles, 0, sizeof(int), st);
+  if (e == cudaSuccess) {
+    nz_tiles<T><<<(unsigned)tiles, kTh, 0, st>>>(val, n, start);
     e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) r = cuda_status(e, "copy_nonzeros");
+  if (!r) r = prim::exclusive_scan(start, start, tiles + 1, st);
+  if (!r) {
+    nz_compact<T><<<(unsigned)tiles, kTh, 0, st>>>(row, col, val, n, start, words,
+                                                   row_ptr ? nullptr : orow_or_ptr, ocol, oval);
+    if (row_ptr)
+      nz_row_ptr<<<g1((long long)N + 1), kTh, 0, st>>>(row_ptr, N, n, words, start + tiles,
+                                                       orow_or_ptr);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) r = cuda_status(e, "copy_nonzeros");
   }
-  if (!r && (e = cudaStreamSynchronize(st)) != cudaSuccess) r = cuda_status(e, "copy_nonzeros");
-  scratch_free(pos, st);
+  scratch_free(mem, st);
   return r;
 }
 
