@@ -121,103 +121,318 @@ __global__ void csr_to_ell(const int* __restrict__ row_ptr, const int* __restric
   }
 }
 
-// Presence of diagonal c - i, stored at index N + c - i - 1 as in the
-// reference (:1498); stores of 1 from several threads are benign.  Rows
-// [r0, r1).  CHECK: a flag is stored only while it reads 0 (a stale 0 costs
-// one more idempotent store).  Every row of a band marks the same few
-// flags, and those repeated stores to a handful of addresses dominated a
-// 4M-row band's conversion (csr_dia 1.17 -> 0.56 ms with the check); with
-// random columns the check is a load round trip in front of every store
-// (a 2M-row power-law num_diags 0.39 -> 0.90 ms), so it is used only where
-// a prefix of the rows spans few diagonals.  SPAN: the prefix pass, which
-// also reduces the smallest and largest N + c - i it marks into span[0]
-// (min) and span[1] (max): one reduction per warp, no returning atomics.
-template <bool CHECK, bool SPAN>
-__global__ void mark_diagonals(const int* __restrict__ row_ptr, const int* __restrict__ col,
-                               int N, int r0, int r1, int* __restrict__ ind,
-                               unsigned* __restrict__ span) {
-  const int i = r0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= r1) return;
-  unsigned lo = 0xffffffffu, hi = 0;
-  for (int j = row_ptr[i]; j < row_ptr[i + 1]; ++j) {
-    const int c = col[j];
-    if (c < 0 || c >= N) continue;
-    const long long d = (long long)N + c - i - 1;
-    int* f = ind + d;
-    if (!CHECK || *f == 0) *f = 1;
-    if (SPAN) {
-      lo = min(lo, (unsigned)d);
-      hi = max(hi, (unsigned)d);
+// The diagonals c - i (c a column within the matrix, i its row) that occur.
+// A stencil's or a band's matrix has few, and its first and last rows show
+// them all: `known_diagonals` collects those of the first and last 512 rows
+// in a hash table, and where they are at most kDiaGather the other rows are
+// only held against that list.  A diagonal outside it (a stray), or a matrix
+// of many, is marked in one byte per diagonal, at N + c - i - 1 as in the
+// reference (:1498), and the bytes are counted and ranked by tiles.
+// A 4M-row band of 9 diagonals on B200, num_diags: one 4-byte flag per
+// diagonal, stored by every row and scanned, 115 us of device time; now 57,
+// 47 of them in mark_diagonals (24 at copy speed for the columns).  csr_dia,
+// which needed the same once more, finds the list in 8 us and checks the
+// entries in its fill.
+constexpr int kDiaGather = 64;
+constexpr int kKnownRows = 512;  // at each end
+
+struct Known {
+  int count;  // of the first and last rows; kDiaGather + 1: more
+  int stray;  // set: a row has a diagonal outside offset[0 .. count)
+  int offset[kDiaGather];
+};
+
+constexpr int kSlots = 256;
+
+__device__ __forceinline__ void insert_offset(int d, int* key, int* count) {
+  unsigned h = ((unsigned)d * 2654435761u) >> 24;
+  for (int step = 0; step < kSlots && *(volatile int*)count <= kDiaGather;
+       ++step, h = (h + 1) & (kSlots - 1)) {
+    int at = *(volatile int*)&key[h];
+    if (at == INT_MAX) {
+      at = atomicCAS(&key[h], INT_MAX, d);
+      if (at == INT_MAX) {
+        atomicAdd(count, 1);
+        return;
+      }
     }
-  }
-  if (SPAN) {
-    const unsigned m = __activemask();
-    lo = __reduce_min_sync(m, lo);
-    hi = __reduce_max_sync(m, hi);
-    if ((threadIdx.x & 31) == __ffs(m) - 1) {
-      atomicMin(span, lo);
-      atomicMax(span + 1, hi);
-    }
+    if (at == d) return;
   }
 }
 
-// Compact the present diagonals: slot[d] = rank of d among present ones
-// (from the exclusive scan), offset[slot] = d - (N - 1) ascending.
-__global__ void compact_diagonals(const int* __restrict__ present, const int* __restrict__ rank,
-                                  long long nd_all, int N, int* __restrict__ offset) {
-  const long long d = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= nd_all) return;
-  if (present[d]) offset[rank[d]] = (int)(d - (N - 1));
+__global__ void __launch_bounds__(2 * kKnownRows)
+    known_diagonals(const int* __restrict__ row_ptr, const int* __restrict__ col, int N,
+                    Known* __restrict__ known) {
+  __shared__ int key[kSlots];
+  __shared__ int count;
+  const int t = threadIdx.x;
+  if (t < kSlots) key[t] = INT_MAX;  // (no diagonal: c - i < N)
+  if (t == 0) count = 0;
+  __syncthreads();
+  const int i = t < kKnownRows ? t : N - 1 - (t - kKnownRows);
+  int s = 0, e = 0;
+  if (t < kKnownRows ? i < N : i >= kKnownRows) {
+    s = row_ptr[i];
+    e = row_ptr[i + 1];
+  }
+  if (e - s > kDiaGather) {
+    atomicAdd(&count, kDiaGather + 1);
+    e = s;
+  }
+  constexpr int kAhead = 8;
+  for (int t0 = 0; t0 < e - s && *(volatile int*)&count <= kDiaGather; t0 += kAhead) {
+    int c[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) c[u] = t0 + u < e - s ? col[s + t0 + u] : -1;
+#pragma unroll 1
+    for (int u = 0; u < kAhead; ++u) {
+      if ((unsigned)c[0] < (unsigned)N) insert_offset(c[0] - i, key, &count);
+#pragma unroll
+      for (int v = 0; v + 1 < kAhead; ++v) c[v] = c[v + 1];
+    }
+  }
+  __syncthreads();
+  const int n = min(count, kDiaGather + 1);
+  if (t == 0) {
+    known->count = n;
+    known->stray = 0;
+  }
+  if (n <= kDiaGather && t < kSlots && key[t] != INT_MAX) {
+    int rank = 0;
+    for (int k = 0; k < kSlots; ++k) rank += key[k] < key[t];
+    known->offset[rank] = key[t];
+  }
+}
+
+// The first of n ascending offsets that is not below d.
+__device__ __forceinline__ int first_place(long long d, const int* off, int n) {
+  int k = 0;
+  while (k < n && off[k] < d) ++k;
+  return k;
+}
+
+// Whether a row's entries (one at least) lie on consecutive offsets, as almost
+// every row of a band or a stencil does.  The loads don't wait on one another.
+__device__ __forceinline__ bool run_of_offsets(const int* __restrict__ col, int s, int e, int i,
+                                               int N, const int* off, int n) {
+  const int k0 = first_place(col[s] - (long long)i, off, n);
+  if (e - s > n - k0) return false;
+  bool ok = true;
+#pragma unroll 8
+  for (int u = 0; u < e - s; ++u) {
+    const int c = col[s + u];
+    ok &= (unsigned)c < (unsigned)N && c - i == off[k0 + u];
+  }
+  return ok;
+}
+
+// Every diagonal of the rows into present: a warp takes `rows` (at most 32)
+// rows at a time and its lanes their entries in storage order, so that loads
+// coalesce and long rows are shared out; an entry's row is found among the
+// row pointers.  Where 32 entries in a row lie on near diagonals (a band, a
+// dense block) a byte is stored only while it reads 0 (a stale 0 costs one
+// more idempotent store), as the same few sectors would otherwise be stored
+// over and over; elsewhere the check would be a round trip for nothing.
+// num_diags on B200, host time: 200k rows of 81 diagonals, checking 0.14 ms,
+// storing plainly 0.30; 2M-row power law of 38M entries 0.56 and 0.44; with
+// 4-byte flags and a thread per row 0.25 and 0.52.
+constexpr int kNarrow = 4096;
+
+__device__ void mark_all(const int* __restrict__ row_ptr, const int* __restrict__ col, int N,
+                         int rows, int (*ptr)[33], unsigned char* present) {
+  const int lane = threadIdx.x & 31;
+  int* p = ptr[threadIdx.x >> 5];
+  const int warps = gridDim.x * (kThreads / 32);
+  const int chunks = (N - 1) / rows + 1;
+  for (int q = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); q < chunks; q += warps) {
+    const int r0 = q * rows, n = min(rows, N - r0);
+    p[lane] = row_ptr[r0 + min(lane, n)];
+    if (lane == 0) p[32] = row_ptr[r0 + n];
+    __syncwarp();
+    const int s = p[0], e = p[32];
+    if (__any_sync(0xffffffffu, p[lane] > p[lane + 1])) {  // row pointers that don't ascend
+      if (lane < n)
+        for (int j = p[lane], end = row_ptr[r0 + lane + 1]; j < end; ++j) {
+          const int c = col[j];
+          if ((unsigned)c < (unsigned)N) present[(long long)N + c - (r0 + lane) - 1] = 1;
+        }
+      __syncwarp();
+      continue;
+    }
+    constexpr int kAhead = 4;
+    const unsigned len = (unsigned)e - (unsigned)s;
+    for (unsigned t0 = 0; t0 < len; t0 += 32 * kAhead) {
+      const unsigned t = t0 + lane;
+      int c[kAhead];
+      long long at[kAhead];  // the byte to set, < 0: none
+      unsigned char have[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) c[u] = t + 32 * u < len ? col[s + t + 32 * u] : -1;
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        int r = 0;  // the last row that begins at or before the entry
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+          if ((unsigned)p[r + step] - (unsigned)s <= t + 32 * u) r += step;
+        at[u] = (unsigned)c[u] < (unsigned)N ? (long long)N + c[u] - (r0 + r) - 1 : -1;
+      }
+      const unsigned lo = __reduce_min_sync(0xffffffffu, at[0] >= 0 ? (unsigned)at[0] : ~0u);
+      const unsigned hi = __reduce_max_sync(0xffffffffu, at[0] >= 0 ? (unsigned)at[0] : 0u);
+      const bool check = hi - lo < (unsigned)kNarrow;
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        have[u] = at[u] >= 0 ? (check ? present[at[u]] : (unsigned char)0) : (unsigned char)1;
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if (!have[u]) present[at[u]] = 1;
+    }
+    __syncwarp();
+  }
+}
+
+// present is zero on entry.
+__global__ void __launch_bounds__(kThreads)
+    mark_diagonals(const int* __restrict__ row_ptr, const int* __restrict__ col, int N, int rows,
+                   Known* __restrict__ known, unsigned char* __restrict__ present) {
+  __shared__ int off[kDiaGather];
+  __shared__ int ptr[kThreads / 32][33];
+  const int n = known->count;
+  if (n > kDiaGather) {
+    mark_all(row_ptr, col, N, rows, ptr, present);
+    return;
+  }
+  if (threadIdx.x < n) {
+    off[threadIdx.x] = known->offset[threadIdx.x];
+    if (blockIdx.x == 0) present[(long long)N + off[threadIdx.x] - 1] = 1;
+  }
+  __syncthreads();
+  bool stray = false;
+  for (long long r = (long long)blockIdx.x * kThreads + threadIdx.x; r < N;
+       r += (long long)gridDim.x * kThreads) {
+    const int i = (int)r, s = row_ptr[i], e = row_ptr[i + 1];
+    if (s >= e || run_of_offsets(col, s, e, i, N, off, n)) continue;
+    for (int j = s; j < e; ++j) {
+      const int c = col[j];
+      if ((unsigned)c >= (unsigned)N) continue;
+      const int k = first_place(c - i, off, n);
+      if (k < n && off[k] == c - i) continue;
+      unsigned char* f = present + ((long long)N + c - i - 1);
+      if (*f == 0) *f = 1;
+      stray = true;
+    }
+  }
+  if (__syncthreads_or(stray) && threadIdx.x == 0) known->stray = 1;
+}
+
+// Counts per tile of 16 bytes a thread, and from the scanned counts the
+// present diagonals' offsets in ascending order and (where asked for) ranks.
+__device__ __forceinline__ int ones(uint4 b) {  // bytes of 0 or 1
+  return __popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w);
+}
+
+__global__ void __launch_bounds__(kThreads)
+    count_bytes(const uint4* __restrict__ present, long long words, int* __restrict__ sums) {
+  const long long w = (long long)blockIdx.x * kThreads + threadIdx.x;
+  __shared__ int total;
+  if (threadIdx.x == 0) total = 0;
+  __syncthreads();
+  const int c = __reduce_add_sync(0xffffffffu, w < words ? ones(present[w]) : 0);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&total, c);
+  __syncthreads();
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kThreads)
+    compact_diagonals(const uint4* __restrict__ present, long long words,
+                      const int* __restrict__ start, int N, int* __restrict__ offset,
+                      int* __restrict__ rank) {
+  __shared__ int warp_sum[kThreads / 32];
+  const long long w = (long long)blockIdx.x * kThreads + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint4 b = w < words ? present[w] : make_uint4(0, 0, 0, 0);
+  const int mine = ones(b);
+  int incl = mine;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += up;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  if (mine == 0) return;
+  int at = start[blockIdx.x] + incl - mine;
+  for (int k = 0; k < warp; ++k) at += warp_sum[k];
+  const unsigned q[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    if ((q[k >> 2] >> (8 * (k & 3)) & 1u) == 0) continue;
+    const long long d = w * 16 + k;
+    offset[at] = (int)(d - (N - 1));
+    if (rank) rank[d] = at;
+    ++at;
+  }
 }
 
 // csr_dia fill for at most kDiaGather diagonals: thread per row; slot k of
 // row i receives the row's LAST entry in column i + offset[k] (the
 // reference's row-major loop, :1559-1571, lets a later duplicate overwrite
-// an earlier one), else +0, so every slot is written exactly once with
-// writes coalesced across rows, and no zero fill or scatter is needed.  Rows
-// of up to kDiaRowRegs entries are held in registers.
-constexpr int kDiaGather = 64;
-constexpr int kDiaRowRegs = 16;
-
-template <typename T>
-__global__ void csr_to_dia_rows(const int* __restrict__ row_ptr, const int* __restrict__ col,
-                                const T* __restrict__ val, int N, int nd,
-                                const int* __restrict__ offset, T* __restrict__ data) {
-  __shared__ int off_s[kDiaGather];
-  for (int k = threadIdx.x; k < nd; k += blockDim.x) off_s[k] = offset[k];
+// an earlier one), else +0, so every slot is written with writes coalesced
+// across rows, and no zero fill or scatter is needed.  A row is taken as a
+// run of consecutive offsets, its loads independent of one another; where
+// that proves wrong its slots are written again by a search per slot.  Loads
+// go in batches of 5 slots (batches of 3 and 8 measured the same, 9 or a plain
+// unrolled loop 9-30% longer).  Comparing 16 entries in registers with every
+// slot took 211 us for a 4M-row FP64 band of 9 diagonals on B200; now 146, at
+// 5.1 TB/s of row pointers, entries and slots.  Entries staged in shared
+// memory measured longer (195).  CHECK: an entry outside the offsets is
+// reported.
+template <typename T, bool CHECK>
+__global__ void __launch_bounds__(kThreads)
+    csr_to_dia_rows(const int* __restrict__ row_ptr, const int* __restrict__ col,
+                    const T* __restrict__ val, int N, int nd, const int* __restrict__ offset,
+                    T* __restrict__ data, int* __restrict__ stray) {
+  __shared__ int off[kDiaGather];
+  const int i = blockIdx.x * kThreads + threadIdx.x;
+  if (threadIdx.x < nd) off[threadIdx.x] = offset[threadIdx.x];
   __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const int s = row_ptr[i], e = row_ptr[i + 1];
-  if (e - s <= kDiaRowRegs) {
-    int rel[kDiaRowRegs];
-    T v[kDiaRowRegs];
+  const int s = row_ptr[i], len = max(row_ptr[i + 1] - s, 0);
+  const int k0 = len > 0 ? first_place(col[s] - (long long)i, off, nd) : 0;
+  bool ok = len <= nd - k0;
+  constexpr int kAhead = 5;
+  for (int kb = 0; kb < nd; kb += kAhead) {
+    int c[kAhead];
+    T v[kAhead];
 #pragma unroll
-    for (int u = 0; u < kDiaRowRegs; ++u) {
-      const bool in = s + u < e;
-      const int c = in ? col[s + u] : -1;
-      // out-of-range columns are not stored (the reference skips them)
-      rel[u] = (in && c >= 0 && c < N) ? c - i : INT_MIN;
-      v[u] = in ? val[s + u] : T(0);
+    for (int u = 0; u < kAhead; ++u) {
+      const int j = kb + u - k0;
+      const bool in = (unsigned)j < (unsigned)len && kb + u < nd;
+      c[u] = in ? col[s + j] : i + off[min(kb + u, nd - 1)];
+      v[u] = in ? val[s + j] : T(0);
+      ok &= !in || (unsigned)c[u] < (unsigned)N;
     }
-    for (int k = 0; k < nd; ++k) {
-      const int want = off_s[k];
-      T out = T(0);
 #pragma unroll
-      for (int u = 0; u < kDiaRowRegs; ++u)
-        if (rel[u] == want) out = v[u];
-      data[(long long)k * N + i] = out;
-    }
-    return;
+    for (int u = 0; u < kAhead; ++u)
+      if (kb + u < nd) {
+        ok &= c[u] - i == off[kb + u];
+        data[(long long)(kb + u) * N + i] = v[u];
+      }
   }
+  if (ok) return;
   for (int k = 0; k < nd; ++k) {
-    const int want = off_s[k];
+    const int want = off[k];
     T out = T(0);
-    for (int j = s; j < e; ++j) {
+    for (int j = s; j < s + len; ++j) {
       const int c = col[j];
-      if (c >= 0 && c < N && c - i == want) out = val[j];
+      // out-of-range columns are not stored (the reference skips them)
+      if ((unsigned)c < (unsigned)N && c - i == want) out = val[j];
     }
     data[(long long)k * N + i] = out;
+  }
+  for (int j = s; CHECK && j < s + len; ++j) {
+    const int c = col[j];
+    if ((unsigned)c >= (unsigned)N) continue;
+    const int k = first_place(c - i, off, nd);
+    if (k == nd || off[k] != c - i) *stray = 1;
   }
 }
 
@@ -340,55 +555,136 @@ static int coo_csr_impl(const int* row, const int* col, const T* val, int N, lon
   return r;
 }
 
-constexpr int kDiaPrefixRows = 4096;   // rows of the counting prefix pass
-constexpr int kDiaFewDiagonals = 64;   // prefix span below this many diagonals: check before storing
+// Presence bytes (a whole number of uint4) and the starts of their tiles, with
+// the total after them.
+struct Diags {
+  long long words, tiles;
+  uint4* present;
+  int* start;
+  Known* known;
+  char* mem;
+};
 
-static int num_diags_impl(const int* row_ptr, const int* col, int N, int** present_out,
-                          int** rank_out, int* nd, cudaStream_t st) {
-  const long long nall = 2LL * N - 1;
-  int* present = nullptr;
-  int r = scratch_alloc((void**)&present, sizeof(int) * (size_t)(2 * nall + 2), st);
+static int diags_alloc(int N, Diags& d, cudaStream_t st) {
+  d.words = (2LL * N - 1 + 15) / 16;
+  d.tiles = (d.words + kThreads - 1) / kThreads;
+  const size_t kb = (sizeof(Known) + 15) & ~(size_t)15;
+  const int r = scratch_alloc((void**)&d.mem, sizeof(uint4) * (size_t)d.words + kb +
+                                                  sizeof(int) * (size_t)(d.tiles + 1), st);
   if (r) return r;
-  int* rank = present + nall;
-  unsigned* span = reinterpret_cast<unsigned*>(rank + nall);  // the allocation's last 2 ints
-  SB_CHECK_CUDA(cudaMemsetAsync(present, 0, sizeof(int) * (size_t)nall, st));
-  SB_CHECK_CUDA(cudaMemsetAsync(span, 0xff, sizeof(unsigned), st));
-  SB_CHECK_CUDA(cudaMemsetAsync(span + 1, 0, sizeof(unsigned), st));
-  // a prefix of the rows, measuring the span of the diagonals it marks: a
-  // narrow span (a band) makes the rest check before storing, a wide one
-  // store plainly
-  const int pre = std::min(N, kDiaPrefixRows);
-  mark_diagonals<false, true><<<grid_for(pre), kThreads, 0, st>>>(row_ptr, col, N, 0, pre,
-                                                                  present, span);
-  SB_CHECK_LAUNCH("mark_diagonals");
-  unsigned hs[2] = {0xffffffffu, 0};
-  SB_CHECK_CUDA(cudaMemcpyAsync(hs, span, sizeof(hs), cudaMemcpyDeviceToHost, st));
-  SB_CHECK_CUDA(cudaStreamSynchronize(st));
-  if (N > pre) {
-    const bool narrow = hs[1] >= hs[0] && hs[1] - hs[0] < (unsigned)kDiaFewDiagonals;
-    if (narrow)
-      mark_diagonals<true, false><<<grid_for(N - pre), kThreads, 0, st>>>(row_ptr, col, N, pre, N,
-                                                                        present, span);
-    else
-      mark_diagonals<false, false><<<grid_for(N - pre), kThreads, 0, st>>>(row_ptr, col, N, pre,
-                                                                         N, present, span);
-    SB_CHECK_LAUNCH("mark_diagonals");
-  }
-  r = prim::exclusive_scan(present, rank, nall, st);
-  if (r) {
-    scratch_free(present, st);
-    return r;
-  }
-  int last[2] = {0, 0};
-  SB_CHECK_CUDA(cudaMemcpyAsync(&last[0], present + nall - 1, sizeof(int),
-                                cudaMemcpyDeviceToHost, st));
-  SB_CHECK_CUDA(cudaMemcpyAsync(&last[1], rank + nall - 1, sizeof(int), cudaMemcpyDeviceToHost,
-                                st));
-  SB_CHECK_CUDA(cudaStreamSynchronize(st));
-  *nd = last[0] + last[1];
-  *present_out = present;
-  *rank_out = rank;
+  d.present = reinterpret_cast<uint4*>(d.mem);
+  d.known = reinterpret_cast<Known*>(d.present + d.words);
+  d.start = reinterpret_cast<int*>(reinterpret_cast<char*>(d.known) + kb);
   return SB_OK;
+}
+
+// The number of diagonals into *nd; all: also the presence bytes and tile
+// starts (left out where the first and last rows show every diagonal).
+static int find_diagonals(const int* row_ptr, const int* col, int N, const Diags& d, bool all,
+                          int* nd, cudaStream_t st) {
+  unsigned char* present = reinterpret_cast<unsigned char*>(d.present);
+  SB_CHECK_CUDA(cudaMemsetAsync(present, 0, sizeof(uint4) * (size_t)d.words, st));
+  known_diagonals<<<1, 2 * kKnownRows, 0, st>>>(row_ptr, col, N, d.known);
+  const unsigned grid = (unsigned)sm_count() * 8;
+  // rows a warp of mark_all takes: as many as leave every warp some, 1 to 32
+  int rows = 32;
+  while (rows > 1 && (long long)rows * grid * (kThreads / 32) > N) rows >>= 1;
+  mark_diagonals<<<grid, kThreads, 0, st>>>(row_ptr, col, N, rows, d.known, present);
+  SB_CHECK_LAUNCH("mark_diagonals");
+  int head[2] = {0, 0};  // known->count, known->stray
+  SB_CHECK_CUDA(cudaMemcpyAsync(head, d.known, sizeof(head), cudaMemcpyDeviceToHost, st));
+  SB_CHECK_CUDA(cudaStreamSynchronize(st));
+  *nd = head[0];
+  if (!all && head[0] <= kDiaGather && !head[1]) return SB_OK;
+  SB_CHECK_CUDA(cudaMemsetAsync(d.start + d.tiles, 0, sizeof(int), st));
+  count_bytes<<<(unsigned)d.tiles, kThreads, 0, st>>>(d.present, d.words, d.start);
+  SB_CHECK_LAUNCH("count_bytes");
+  const int r = prim::exclusive_scan(d.start, d.start, d.tiles + 1, st);
+  if (r) return r;
+  SB_CHECK_CUDA(cudaMemcpyAsync(nd, d.start + d.tiles, sizeof(int), cudaMemcpyDeviceToHost, st));
+  SB_CHECK_CUDA(cudaStreamSynchronize(st));
+  return SB_OK;
+}
+
+static int num_diags_impl(const int* row_ptr, const int* col, int N, int* nd, cudaStream_t st) {
+  Diags d;
+  int r = diags_alloc(N, d, st);
+  if (r) return r;
+  r = find_diagonals(row_ptr, col, N, d, false, nd, st);
+  scratch_free(d.mem, st);
+  return r;
+}
+
+// csr_dia of a matrix whose first and last rows show all of its nd diagonals:
+// *done set once the arrays are complete.  The fill itself checks every entry.
+template <typename T>
+static int csr_dia_known(const int* row_ptr, const int* col, const T* val, int N, int nd,
+                         int* offset, T* data, bool* done, cudaStream_t st) {
+  *done = false;
+  Known* known = nullptr;
+  int r = scratch_alloc((void**)&known, sizeof(Known), st);
+  if (r) return r;
+  int head[2] = {0, 0};
+  known_diagonals<<<1, 2 * kKnownRows, 0, st>>>(row_ptr, col, N, known);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(head, known, sizeof(head), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess && head[0] == nd && nd <= kDiaGather) {
+    e = cudaMemcpyAsync(offset, known->offset, sizeof(int) * (size_t)nd, cudaMemcpyDeviceToDevice,
+                        st);
+    if (e == cudaSuccess) {
+      csr_to_dia_rows<T, true><<<grid_for(N), kThreads, 0, st>>>(row_ptr, col, val, N, nd,
+                                                                known->offset, data, &known->stray);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(head, known, sizeof(head), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    *done = e == cudaSuccess && !head[1];
+  }
+  scratch_free(known, st);
+  return e == cudaSuccess ? SB_OK : cuda_status(e, "sb_csr_dia");
+}
+
+template <typename T>
+static int csr_dia_impl(const int* row_ptr, const int* col, const T* val, int N, int nd,
+                        int stride, int* offset, T* data, cudaStream_t st) {
+  bool done = false;
+  int r = csr_dia_known(row_ptr, col, val, N, nd, offset, data, &done, st);
+  if (r || done) return r;
+  Diags d;
+  if ((r = diags_alloc(N, d, st))) return r;
+  int* rank = nullptr;
+  int nd_found = 0;
+  r = find_diagonals(row_ptr, col, N, d, true, &nd_found, st);
+  if (!r && nd_found != nd) {
+    set_error("sb_csr_dia: nd=%d does not match the matrix (%d diagonals)", nd, nd_found);
+    r = SB_EINVAL;
+  }
+  if (!r && nd > kDiaGather)
+    r = scratch_alloc((void**)&rank, sizeof(int) * (size_t)(2LL * N - 1), st);
+  if (!r) {
+    compact_diagonals<<<(unsigned)d.tiles, kThreads, 0, st>>>(d.present, d.words, d.start, N,
+                                                              offset, rank);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess && nd <= kDiaGather) {
+      // gather: every slot written once (stride == N)
+      csr_to_dia_rows<T, false><<<grid_for(N), kThreads, 0, st>>>(row_ptr, col, val, N, nd, offset,
+                                                                 data, nullptr);
+      e = cudaGetLastError();
+    } else if (e == cudaSuccess) {
+      e = cudaMemsetAsync(data, 0, sizeof(T) * (size_t)nd * (size_t)stride, st);
+      if (e == cudaSuccess) {
+        csr_to_dia<T><<<grid_for(N), kThreads, 0, st>>>(row_ptr, col, val, N, stride, rank, data);
+        e = cudaGetLastError();
+      }
+    }
+    if (e != cudaSuccess) r = cuda_status(e, "sb_csr_dia");
+  }
+  if (rank) scratch_free(rank, st);
+  scratch_free(d.mem, st);
+  return r;
 }
 
 }  // namespace sb
@@ -481,10 +777,7 @@ int sb_num_diags(const int32_t* row_ptr, const int32_t* col, int32_t N, int32_t*
   int r = ensure_device();
   if (r) return r;
   cudaStream_t st = as_stream(stream);
-  int *present = nullptr, *rank = nullptr;
-  if ((r = num_diags_impl(row_ptr, col, N, &present, &rank, nd, st))) return r;
-  scratch_free(present, st);
-  return SB_OK;
+  return num_diags_impl(row_ptr, col, N, nd, st);
 }
 
 int sb_dia_admitted(int64_t ndiags, int32_t stride, int64_t nnz) {
@@ -507,41 +800,10 @@ int sb_csr_dia(int dtype, const int32_t* row_ptr, const int32_t* col, const void
   SB_REQUIRE(row_ptr && col && val && offset && data, "sb_csr_dia: null pointer");
   if ((r = ensure_device())) return r;
   cudaStream_t st = as_stream(stream);
-  int *present = nullptr, *rank = nullptr;
-  int nd_found = 0;
-  if ((r = num_diags_impl(row_ptr, col, N, &present, &rank, &nd_found, st))) return r;
-  if (nd_found != nd) {
-    scratch_free(present, st);
-    set_error("sb_csr_dia: nd=%d does not match the matrix (%d diagonals)", nd, nd_found);
-    return SB_EINVAL;
-  }
-  const long long nall = 2LL * N - 1;
-  compact_diagonals<<<grid_for(nall), kThreads, 0, st>>>(present, rank, nall, N, offset);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess && nd <= kDiaGather) {
-    // gather: every slot written once (stride == N)
-    if (dtype == SB_F32)
-      csr_to_dia_rows<float><<<grid_for(N), kThreads, 0, st>>>(
-          row_ptr, col, (const float*)val, N, nd, offset, (float*)data);
-    else
-      csr_to_dia_rows<double><<<grid_for(N), kThreads, 0, st>>>(
-          row_ptr, col, (const double*)val, N, nd, offset, (double*)data);
-    e = cudaGetLastError();
-  } else if (e == cudaSuccess) {
-    e = cudaMemsetAsync(data, 0, dtype_size(dtype) * (size_t)nd * (size_t)stride, st);
-    if (e == cudaSuccess) {
-      if (dtype == SB_F32)
-        csr_to_dia<float><<<grid_for(N), kThreads, 0, st>>>(row_ptr, col, (const float*)val, N,
-                                                            stride, rank, (float*)data);
-      else
-        csr_to_dia<double><<<grid_for(N), kThreads, 0, st>>>(row_ptr, col, (const double*)val, N,
-                                                             stride, rank, (double*)data);
-      e = cudaGetLastError();
-    }
-  }
-  scratch_free(present, st);
-  if (e != cudaSuccess) return cuda_status(e, "sb_csr_dia");
-  return SB_OK;
+  return dtype == SB_F32 ? csr_dia_impl<float>(row_ptr, col, (const float*)val, N, nd, stride,
+                                               offset, (float*)data, st)
+                         : csr_dia_impl<double>(row_ptr, col, (const double*)val, N, nd, stride,
+                                                offset, (double*)data, st);
 }
 
 int sb_coo_csc(int dtype, const int32_t* row, const int32_t* col, const void* val, int32_t N,
