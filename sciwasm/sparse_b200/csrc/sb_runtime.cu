@@ -21,6 +21,7 @@ void set_error(const char* fmt, ...) {
 }
 
 int cuda_status(cudaError_t e, const char* what) {
+  cudaGetLastError();  // reported here, not again at the next launch
   set_error("%s: %s (%s)", what, cudaGetErrorName(e), cudaGetErrorString(e));
   if (e == cudaErrorMemoryAllocation) return SB_ENOMEM;
   if (e == cudaErrorNoDevice || e == cudaErrorInsufficientDriver) return SB_ENODEV;
@@ -97,7 +98,7 @@ static void keep_pool_memory() {
 // the arrays of a conversion, and differ from call to call.  Freed blocks are
 // therefore kept, up to kPoolKeep bytes per device (the oldest go first), and
 // handed out again for the same (rounded) size.  csr_dia and csr_ell of a 44M-entry
-// FP64 matrix on B200: 3.3 ms and more in all, 0.7 of it kernels; now 0.80.
+// FP64 matrix on B200: 3.3 ms and more in all, 0.80 with the same kernels.
 // Level sets with reordering of a 1M-row factor 6.9 -> 2.5 ms.
 //   * A block may still be in use by work in flight on any stream when it is
 //     freed (cudaFree would wait for that).  It is handed out again only after

@@ -103,3 +103,12 @@ def test_threads(gpu):
     for t in ts:
         t.join()
     assert not bad
+
+
+def test_refused_allocation_is_reported_once(gpu):
+    """The launch check of the next call must not see the old error."""
+    _, total = _info()
+    q = ctypes.c_void_p()
+    assert _lib.load().sb_malloc(ctypes.byref(q), total * 2) == _lib.SB_ENOMEM
+    A = gpu.csr_from_host(np.array([0, 1, 2]), np.array([0, 1]), np.array([0.0, 3.0]))
+    assert gpu.eliminate_zeros(A).nnz == 1
