@@ -128,9 +128,9 @@ __global__ void csr_to_ell(const int* __restrict__ row_ptr, const int* __restric
 // only held against that list.  A diagonal outside it (a stray), or a matrix
 // of many, is marked in one byte per diagonal, at N + c - i - 1 as in the
 // reference (:1498), and the bytes are counted and ranked by tiles.
-// A 4M-row band of 9 diagonals on B200, num_diags: one 4-byte flag per
+// A 4M-row band of 11 diagonals on B200, num_diags: one 4-byte flag per
 // diagonal, stored by every row and scanned, 115 us of device time; now 57,
-// 47 of them in mark_diagonals (24 at copy speed for the columns).  csr_dia,
+// 47 of them in mark_diagonals (29 at copy speed for the columns).  csr_dia,
 // which needed the same once more, finds the list in 8 us and checks the
 // entries in its fill.
 constexpr int kDiaGather = 64;
@@ -381,8 +381,8 @@ __global__ void __launch_bounds__(kThreads)
 // that proves wrong its slots are written again by a search per slot.  Loads
 // go in batches of 5 slots (batches of 3 and 8 measured the same, 9 or a plain
 // unrolled loop 9-30% longer).  Comparing 16 entries in registers with every
-// slot took 211 us for a 4M-row FP64 band of 9 diagonals on B200; now 146, at
-// 5.1 TB/s of row pointers, entries and slots.  Entries staged in shared
+// slot took 211 us for a 4M-row FP64 band of 11 diagonals on B200; now 146, at
+// 6.1 TB/s of row pointers, entries and slots.  Entries staged in shared
 // memory measured longer (195).  CHECK: an entry outside the offsets is
 // reported.
 template <typename T, bool CHECK>
