@@ -96,20 +96,30 @@ static void keep_pool_memory() {
 // ---------------------------------------------------------------- device memory
 // cudaMalloc and cudaFree map and unmap pages: 0.1 to several milliseconds for
 // the arrays of a conversion, and differ from call to call.  Freed blocks are
-// therefore kept, up to kPoolKeep bytes per device (the oldest go first), and
+// therefore kept, up to kKeepBytes per device (the oldest go first), and
 // handed out again for the same (rounded) size.  csr_dia and csr_ell of a 44M-entry
 // FP64 matrix on B200: 3.3 ms and more in all, 0.80 with the same kernels.
 // Level sets with reordering of a 1M-row factor 6.9 -> 2.5 ms.
 //   * A block may still be in use by work in flight on any stream when it is
-//     freed (cudaFree would wait for that).  It is handed out again only after
-//     the device has been synchronised since; where that fails (a stream is
-//     being captured) a fresh block is taken.
+//     freed.  It is handed out again only after a cudaFree since, which waits for
+//     that work as the free of the block itself would have.  (A device
+//     synchronisation waits too, in 3 us against 0.66 ms for a small cudaMalloc
+//     and cudaFree, but it invalidates a stream capture that another thread has
+//     under way, or this one in relaxed mode; cudaMalloc and cudaFree don't.)
+//     One wait serves all blocks freed before it, so new blocks are taken while
+//     little is kept (kEnoughBytes, and kEnoughSame blocks of one size), and only
+//     then does an allocation wait.
 //   * Kept blocks are given back to the driver when an allocation of this
 //     library fails, before it is tried once more; sb_mem_info counts them as
 //     free.
 //   * Pointers that did not come from here go to cudaFree as they are; freeing a
 //     kept block again is an error, as it is for cudaFree.
 namespace {
+
+constexpr size_t kKeepBytes = 4ull << 30;
+constexpr size_t kEnoughBytes = 3ull << 30;
+constexpr size_t kEnoughSame = 16;
+constexpr size_t kKeepBlocks = 2048;
 
 struct Block {
   void* ptr;
@@ -120,7 +130,7 @@ struct Block {
 struct Pool {
   std::list<Block> kept;  // oldest first
   size_t kept_bytes = 0;
-  uint64_t synced = 0;  // the clock when the device was last synchronised here
+  uint64_t synced = 0;  // the clock when a wait for the device's work last ended
 };
 
 struct Memory {
@@ -143,9 +153,21 @@ size_t round_size(size_t b) {
   return (b + step - 1) / step * step;
 }
 
-// Gives the pool's blocks back to the driver until at most `most` bytes are kept.
-void trim(Pool& pool, size_t most) {
-  while (pool.kept_bytes > most) {
+// Waits for the work that may use the kept blocks.
+bool wait_for_uses(Pool& pool, Memory& mem) {
+  void* p = nullptr;
+  if (cudaMalloc(&p, 16) != cudaSuccess || cudaFree(p) != cudaSuccess) {
+    cudaGetLastError();  // the allocation that follows reports what is wrong
+    return false;
+  }
+  pool.synced = ++mem.clock;
+  return true;
+}
+
+// Gives the pool's blocks back to the driver, the oldest first, until at most
+// `most` bytes in `blocks` blocks are kept.
+void trim(Pool& pool, size_t most, size_t blocks) {
+  while (pool.kept_bytes > most || pool.kept.size() > blocks) {
     cudaFree(pool.kept.front().ptr);
     pool.kept_bytes -= pool.kept.front().bytes;
     pool.kept.pop_front();
@@ -165,25 +187,26 @@ int device_alloc(void** p, size_t bytes) {
   std::lock_guard<std::mutex> lk(mem.mu);
   Pool& pool = mem.pools[dev];
   // the block of this very size that was freed first
+  size_t same = 0;
+  auto first = pool.kept.end();
   for (auto it = pool.kept.begin(); it != pool.kept.end(); ++it) {
     if (it->bytes != want) continue;
-    if (it->freed > pool.synced) {
-      if (cudaDeviceSynchronize() != cudaSuccess) {
-        cudaGetLastError();  // cudaMalloc reports what is wrong, if it is
-        break;
-      }
-      pool.synced = ++mem.clock;
-    }
-    *p = it->ptr;
-    pool.kept_bytes -= it->bytes;
-    pool.kept.erase(it);
+    if (same++ == 0) first = it;
+    if (it->freed <= pool.synced) break;
+  }
+  if (same && (first->freed <= pool.synced ||
+               ((pool.kept_bytes >= kEnoughBytes || same >= kEnoughSame) &&
+                wait_for_uses(pool, mem)))) {
+    *p = first->ptr;
+    pool.kept_bytes -= first->bytes;
+    pool.kept.erase(first);
     mem.live[*p] = {want, dev};
     return SB_OK;
   }
   e = cudaMalloc(p, want);
   if (e == cudaErrorMemoryAllocation && pool.kept_bytes) {
     cudaGetLastError();
-    trim(pool, 0);
+    trim(pool, 0, 0);
     e = cudaMalloc(p, want);
   }
   if (e != cudaSuccess) {
@@ -209,11 +232,11 @@ int device_free(void* p) {
   const size_t bytes = it->second.first;
   Pool& pool = mem.pools[it->second.second];
   mem.live.erase(it);
-  if (bytes > kPoolKeep) {
+  if (bytes > kKeepBytes) {
     SB_CHECK_CUDA(cudaFree(p));
     return SB_OK;
   }
-  trim(pool, kPoolKeep - bytes);
+  trim(pool, kKeepBytes - bytes, kKeepBlocks - 1);
   pool.kept.push_back({p, bytes, ++mem.clock});
   pool.kept_bytes += bytes;
   return SB_OK;
@@ -232,7 +255,7 @@ int scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
     std::lock_guard<std::mutex> lk(mem.mu);
     if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 &&
         mem.pools[dev].kept_bytes) {
-      trim(mem.pools[dev], 0);
+      trim(mem.pools[dev], 0, 0);
       e = cudaMallocAsync(p, bytes, s);
     }
   }

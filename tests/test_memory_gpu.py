@@ -29,7 +29,8 @@ def _info():
 
 def test_reuse_waits_for_the_old_use(gpu):
     """A long chain of copies out of a block on one stream; the block is freed
-    and allocated again meanwhile, and overwritten on another stream."""
+    and allocations of its size follow meanwhile until one gets it, which is
+    overwritten on another stream."""
     n = 256 * MIB
     streams = []
     for _ in range(2):
@@ -37,22 +38,63 @@ def test_reuse_waits_for_the_old_use(gpu):
         _lib.call("sb_stream_create", ctypes.byref(s))
         streams.append(s.value)
     src, dst = _alloc(n), _alloc(n)
+    others = [_alloc(n) for _ in range(16)]
+    _lib.call("sb_stream_synchronize", streams[0])
     _lib.call("sb_memset", src, 0x5A, n, streams[0])
     for _ in range(40):
         _lib.call("sb_memcpy_dtod", dst, src, n, streams[0])
-    _lib.call("sb_free", src)
-    again = _alloc(n)
-    _lib.call("sb_memset", again, 0, n, streams[1])
+    for p in [src] + others:
+        _lib.call("sb_free", p)
+    got = []
+    while src not in got and len(got) < 64:
+        got.append(_alloc(n))
+    _lib.call("sb_memset", got[-1], 0, n, streams[1])
     _lib.call("sb_stream_synchronize", streams[0])
     _lib.call("sb_stream_synchronize", streams[1])
     out = np.empty(n, np.uint8)
     _lib.call("sb_memcpy_dtoh", out.ctypes.data, dst, n, None)
     _lib.call("sb_stream_synchronize", None)
-    assert again == src and np.all(out == 0x5A)
-    for p in (again, dst):
+    assert np.all(out == 0x5A)
+    for p in got + [dst]:
         _lib.call("sb_free", p)
     for s in streams:
         _lib.call("sb_stream_destroy", s)
+
+
+@pytest.mark.parametrize("mode", ["relaxed", "thread_local"])
+def test_allocation_beside_a_capture(gpu, mode):
+    """Blocks are freed and allocated, reused ones too, by this thread while
+    another thread captures a stream (thread_local) or this one does (relaxed):
+    the capture stays valid."""
+    torch = pytest.importorskip("torch")
+    n, x = 64 * MIB, torch.zeros(1000, device="cuda")
+    g, begun, done = torch.cuda.CUDAGraph(), threading.Event(), threading.Event()
+    seen = []
+
+    def churn():
+        for _ in range(60):
+            seen.append(_alloc(n))
+            _lib.call("sb_free", seen[-1])
+
+    def capture(inside):
+        with torch.cuda.graph(g, capture_error_mode=mode):
+            x.add_(1)
+            begun.set()
+            inside()
+            x.add_(1)
+
+    if mode == "relaxed":
+        capture(churn)
+    else:
+        t = threading.Thread(target=capture, args=(lambda: done.wait(60),))
+        t.start()
+        begun.wait(60)
+        churn()
+        done.set()
+        t.join()
+    g.replay()
+    torch.cuda.synchronize()
+    assert len(set(seen)) < len(seen) and torch.all(x == 2)
 
 
 def test_double_free_and_distinct_blocks(gpu):
