@@ -415,7 +415,8 @@ __device__ __forceinline__ void solve_rows(const View<T>& f, T* ring, uint64_t* 
     const bool on = lane < group_rows(g0);
     const int slot = slot0 + lane < f.window ? slot0 + lane : slot0 + lane - f.window;
     if (on) ring[slot] = yi;
-    if (!__all_sync(0xffffffffu, open)) return;  // (and orders the ring's stores)
+    if (!__all_sync(0xffffffffu, open)) return;
+    __syncwarp();  // the lanes' ring stores before lane 0's arrival (a vote orders no memory)
     if (lane == 0) arrive_count(done + g0.z % kLevelBars, group_arrivals(g0));
     if (on) __stcg(f.yw + g0.x + lane, yi);
     slot0 += g1.x - g0.x;

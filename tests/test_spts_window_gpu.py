@@ -105,3 +105,39 @@ def test_window_solves_bitexact(gpu, oracle, dt):
             for (name, want), job in list(zip(wants, run))[pick]:
                 assert np.array_equal(_ub(job[2].to_host()), _ub(want)), (name, pick)
         e.close()
+
+
+@pytest.mark.parametrize("dt,policy", [(np.float32, "native"), (np.float32, "f64"),
+                                       (np.float64, "native")])
+def test_window_solves_special_values(gpu, oracle, dt, policy):
+    """Every lane's value is published before its level closes, and values pass
+    as they are: infinities and NaN in b and L, zero diagonals (0/0, x/0) in rows
+    that others read beside rows padded to their group's length.  Same results
+    run after run; NaNs where the oracle has them, other values bit for bit."""
+    rng = np.random.default_rng(11)
+    rp, col, val = _levels([33, 70, 31, 64, 5] * 30, 7, 3, dt, seed=8)
+    N = rp.size - 1
+    b = synth.uniform_vec(N, 6, dtype=dt)
+    b[rng.integers(0, N, 6)] = [np.inf, -np.inf, np.nan, -0.0, 0.0, np.inf]
+    off = np.setdiff1d(np.arange(val.size), rp[1:] - 1)
+    val[rng.choice(off, 4, replace=False)] = [np.inf, -np.inf, np.nan, -0.0]
+    val[rp[rng.integers(N // 2, N, 3) + 1] - 1] = [0.0, -0.0, np.inf]
+    with np.errstate(all="ignore"):
+        if policy == "native":
+            want = oracle.spts_csr(rp, col, val, b)
+        else:  # sums in FP64, each value rounded to FP32 once
+            want = np.empty(N, np.float32)
+            for i in range(N):
+                s, e = rp[i], rp[i + 1] - 1
+                t = np.float64(0)
+                for j in range(s, e):
+                    t = t + np.float64(val[j]) * np.float64(want[col[j]])
+                want[i] = np.float32((np.float64(b[i]) - t) / np.float64(val[e]))
+    assert np.isnan(want).any() and np.isinf(want).any() and np.isfinite(want).sum() > N // 10
+    A, bv, yv = gpu.csr_from_host(rp, col, val), gpu.vec_from_host(b), gpu.create_vec(N, 0, dt)
+    nan = np.isnan(want)
+    for _ in range(20):
+        gpu.spts(A, bv, yv, algo="hybrid", policy=policy)
+        y = yv.array()
+        assert np.array_equal(np.isnan(y), nan)
+        assert np.array_equal(_ub(y[~nan]), _ub(want[~nan]))
