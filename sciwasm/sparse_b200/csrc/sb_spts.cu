@@ -1205,7 +1205,7 @@ static int analyze_impl(sb_spts_plan* p, cudaStream_t st) {
       if (!r) {
         win::window_fill<T><<<grid1(N), kT, 0, st>>>(
             p->row_ptr, p->col, (const T*)p->val, p->perm, p->order, p->level, p->level_ptr, gstart,
-            glen, gbase, N, L, gmax, cap, h.lower_bad == 0, info, groups, p->records);
+            glen, gbase, N, L, cap, h.lower_bad == 0, info, groups, p->records);
         e = cudaGetLastError();
         if (e != cudaSuccess) r = cuda_status(e, "window_fill");
       }

@@ -67,12 +67,13 @@ constexpr int kSmem = 225 * 1024;  // ring and stages, of the 227 KB a block may
 struct Info {
   int reach;   // rows from a dependency to the end of the level that reads it, at most
   int kmax;    // longest row, off-diagonal entries
-  int size16;  // 16-byte units of all group records
   int use;
   int window;  // ring slots
   int widest;  // groups of a level at most
   int rows;    // rows of a level at most
   int ngroups;
+  unsigned long long size16;  // 16-byte units of all group records, also where they
+                              // are too many for the layout's 32-bit offsets
 };
 
 // A group: {first row, record offset in 16-byte units, level,
@@ -152,16 +153,20 @@ __global__ void window_lengths(const int* __restrict__ row_ptr, const int* __res
 }
 
 // Record sizes (n = the bound on the number of groups; those past the last
-// have none), to be scanned; the longest row into info.
+// have none), to be scanned; their total and the longest row into info.
 __global__ void window_sizes(const int4* __restrict__ groups, const int* __restrict__ glen, int n,
                              const int* __restrict__ ngroups, int tsize, int* __restrict__ size,
                              Info* __restrict__ info) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g > n) return;
-  const bool in = g < *ngroups;
+  const bool in = g <= n && g < *ngroups;
   const int k = in ? glen[g] : 0;
-  size[g] = in ? record16(group_rows(groups[g]), min(k, kMaxK), tsize) : 0;
-  if (k > 0) atomicMax(&info->kmax, k);
+  const int units = in ? record16(group_rows(groups[g]), min(k, kMaxK), tsize) : 0;
+  if (g <= n) size[g] = units;
+  const int sum = __reduce_add_sync(0xffffffffu, units), most = __reduce_max_sync(0xffffffffu, k);
+  if ((threadIdx.x & 31) == 0) {
+    if (sum) atomicAdd(&info->size16, (unsigned long long)sum);
+    if (most > 0) atomicMax(&info->kmax, most);
+  }
 }
 
 // Values of a row that the solve holds in registers (the diagonal and up to
@@ -170,42 +175,42 @@ __host__ __device__ __forceinline__ int unroll_of(int kmax) {
   return kmax <= 3 ? 4 : kmax <= 7 ? 8 : 16;
 }
 
-// Whether to build the layout: it fits (size16: the record units, cap: the
-// units there is room for; lower: the structure the solves need), and one
-// block with its window solves the factor faster than ready flags over the
-// whole GPU.  A block takes a fixed time per group once a level has several,
-// the ready flags a fixed time per level.  Measured on B200 (ns per group at
-// KU 4 / 8 / 16: FP32 24 / 35 / 75, FP64 27 / 51 / 105; us per level of the
-// ready flags: FP32 1.05-1.14, FP64 1.26-1.35), the two meet at about 40, 26
-// and 12 groups per level.
-__device__ __forceinline__ int window_rows(int reach) {
-  return max(kGroup, (reach + kGroup - 1) / kGroup * kGroup);
+// Whether to build the layout: it fits (cap: the record units there is room
+// for, below 2^30, so that offsets into accepted ones fit in 32 bits, while the
+// total can pass 2^31 from 215M FP64 rows on; lower: the structure the solves
+// need), and one block with its window solves the factor faster than ready
+// flags over the whole GPU.  A block takes a fixed time per group once a level
+// has several, the ready flags a fixed time per level.  Measured on B200 (ns
+// per group at KU 4 / 8 / 16: FP32 24 / 35 / 75, FP64 27 / 51 / 105; us per
+// level of the ready flags: FP32 1.05-1.14, FP64 1.26-1.35), the two meet at
+// about 40, 26 and 12 groups per level.
+__host__ __device__ __forceinline__ int window_rows(int reach) {
+  return reach > kGroup ? (reach + kGroup - 1) / kGroup * kGroup : kGroup;
 }
-__device__ __forceinline__ bool window_wins(const Info& f, int size16, int ngroups, int nlevels,
-                                            long long cap, int tsize, bool lower) {
+__host__ __device__ __forceinline__ bool window_wins(const Info& f, int ngroups, int nlevels,
+                                                     long long cap, int tsize, bool lower) {
   const int w = window_rows(f.reach), u = unroll_of(f.kmax);
   const int most = u == 4 ? 40 : u == 8 ? 26 : 12;
-  return lower && w <= 0xffff && f.kmax <= kMaxK && size16 <= cap && f.widest <= kMaxArrivals &&
-         smem_bytes(w, tsize) <= kSmem && (long long)ngroups <= (long long)most * nlevels;
+  return lower && f.reach < 0xffe0 && f.kmax <= kMaxK && (long long)f.size16 <= cap &&
+         f.widest <= kMaxArrivals && smem_bytes(w, tsize) <= kSmem &&
+         (long long)ngroups <= (long long)most * nlevels;
 }
 
 // Decides, completes the group descriptors and writes the records: one thread
-// per row in level order (gmax: the bound on the number of groups).
+// per row in level order.
 template <typename T>
 __global__ void window_fill(const int* __restrict__ row_ptr, const int* __restrict__ col,
                             const T* __restrict__ val, const int* __restrict__ perm,
                             const int* __restrict__ order, const int* __restrict__ level,
                             const int* __restrict__ level_ptr, const int* __restrict__ gstart,
                             const int* __restrict__ glen, const int* __restrict__ gbase, int N,
-                            int nlevels, int gmax, long long cap, bool lower, Info* info,
+                            int nlevels, long long cap, bool lower, Info* info,
                             int4* __restrict__ groups, char* __restrict__ records) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= N) return;
-  const bool use =
-      window_wins(*info, gbase[gmax], gstart[nlevels], nlevels, cap, sizeof(T), lower);
+  const bool use = window_wins(*info, gstart[nlevels], nlevels, cap, sizeof(T), lower);
   const int w = window_rows(info->reach);
   if (p == 0) {
-    info->size16 = gbase[gmax];
     info->ngroups = gstart[nlevels];
     info->window = w;
     info->use = use;
