@@ -1,13 +1,11 @@
 // sb_runtime.cu -- device memory, streams and error reporting of the C ABI.
 // Stands in for MatMachJS's _malloc/_free over wasm linear memory
 // (src/sequential/libs/matmachjs.wat:46-48) with device memory.
-#include <algorithm>
-#include <list>
 #include <mutex>
 #include <string.h>
-#include <unordered_map>
 
 #include "sb_common.cuh"
+#include "sb_kept_blocks.cuh"
 
 namespace sb {
 
@@ -94,84 +92,27 @@ static void keep_pool_memory() {
 }
 
 // ---------------------------------------------------------------- device memory
-// cudaMalloc and cudaFree map and unmap pages: 0.1 to several milliseconds for
-// the arrays of a conversion, and differ from call to call.  Freed blocks are
-// therefore kept, up to kKeepBytes per device (the oldest go first), and
-// handed out again for the same (rounded) size.  csr_dia and csr_ell of a 44M-entry
-// FP64 matrix on B200: 3.3 ms and more in all, 0.80 with the same kernels.
-// Level sets with reordering of a 1M-row factor 6.9 -> 2.5 ms.
-//   * A block may still be in use by work in flight on any stream when it is
-//     freed.  It is handed out again only after a cudaFree since, which waits for
-//     that work as the free of the block itself would have.  (A device
-//     synchronisation waits too, in 3 us against 0.66 ms for a small cudaMalloc
-//     and cudaFree, but it invalidates a stream capture that another thread has
-//     under way, or this one in relaxed mode; cudaMalloc and cudaFree don't.)
-//     One wait serves all blocks freed before it, so new blocks are taken while
-//     little is kept (kEnoughBytes, and kEnoughSame blocks of one size), and only
-//     then does an allocation wait.
-//   * Kept blocks are given back to the driver when an allocation of this
-//     library fails, before it is tried once more; sb_mem_info counts them as
-//     free.
-//   * Pointers that did not come from here go to cudaFree as they are; freeing a
-//     kept block again is an error, as it is for cudaFree.
 namespace {
 
-constexpr size_t kKeepBytes = 4ull << 30;
-constexpr size_t kEnoughBytes = 3ull << 30;
-constexpr size_t kEnoughSame = 16;
-constexpr size_t kKeepBlocks = 2048;
-
-struct Block {
-  void* ptr;
-  size_t bytes;
-  uint64_t freed;  // the pool's clock when it was freed
+struct CudaApi {
+  using Error = cudaError_t;
+  static Error malloc(void** p, size_t bytes) { return cudaMalloc(p, bytes); }
+  static Error free(void* p) { return cudaFree(p); }
+  static Error out_of_memory() { return cudaErrorMemoryAllocation; }
+  static void clear() { cudaGetLastError(); }
 };
 
-struct Pool {
-  std::list<Block> kept;  // oldest first
-  size_t kept_bytes = 0;
-  uint64_t synced = 0;  // the clock when a wait for the device's work last ended
-};
-
-struct Memory {
-  std::mutex mu;
-  uint64_t clock = 0;
-  Pool pools[64];
-  std::unordered_map<void*, std::pair<size_t, int>> live;  // pointer -> (bytes, device)
-};
 // Never destroyed: objects may still be freed while the process ends.
-Memory& memory() {
-  static Memory* m = new Memory;
+KeptBlocks<CudaApi>& memory() {
+  static auto* m = new KeptBlocks<CudaApi>;
   return *m;
 }
 
-// Sizes are rounded so that nearly equal requests share a block: up by at most
-// 1/64, to a multiple of 512 bytes, and by less than 2 MiB (a page).
-size_t round_size(size_t b) {
-  size_t step = 512;
-  while (step < (2u << 20) && step * 128 <= b) step <<= 1;
-  return (b + step - 1) / step * step;
-}
-
-// Waits for the work that may use the kept blocks.
-bool wait_for_uses(Pool& pool, Memory& mem) {
-  void* p = nullptr;
-  if (cudaMalloc(&p, 16) != cudaSuccess || cudaFree(p) != cudaSuccess) {
-    cudaGetLastError();  // the allocation that follows reports what is wrong
-    return false;
-  }
-  pool.synced = ++mem.clock;
-  return true;
-}
-
-// Gives the pool's blocks back to the driver, the oldest first, until at most
-// `most` bytes in `blocks` blocks are kept.
-void trim(Pool& pool, size_t most, size_t blocks) {
-  while (pool.kept_bytes > most || pool.kept.size() > blocks) {
-    cudaFree(pool.kept.front().ptr);
-    pool.kept_bytes -= pool.kept.front().bytes;
-    pool.kept.pop_front();
-  }
+int current_device(int* dev) {
+  const cudaError_t e = cudaGetDevice(dev);
+  if (e != cudaSuccess || *dev < 0 || *dev >= KeptBlocks<CudaApi>::kDevices)
+    return cuda_status(e == cudaSuccess ? cudaErrorInvalidDevice : e, "cudaGetDevice");
+  return SB_OK;
 }
 
 }  // namespace
@@ -179,67 +120,18 @@ void trim(Pool& pool, size_t most, size_t blocks) {
 int device_alloc(void** p, size_t bytes) {
   *p = nullptr;
   int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess || dev < 0 || dev >= 64)
-    return cuda_status(e == cudaSuccess ? cudaErrorInvalidDevice : e, "cudaGetDevice");
-  const size_t want = round_size(std::max<size_t>(bytes, 16));
-  Memory& mem = memory();
-  std::lock_guard<std::mutex> lk(mem.mu);
-  Pool& pool = mem.pools[dev];
-  // the block of this very size that was freed first
-  size_t same = 0;
-  auto first = pool.kept.end();
-  for (auto it = pool.kept.begin(); it != pool.kept.end(); ++it) {
-    if (it->bytes != want) continue;
-    if (same++ == 0) first = it;
-    if (it->freed <= pool.synced) break;
-  }
-  if (same && (first->freed <= pool.synced ||
-               ((pool.kept_bytes >= kEnoughBytes || same >= kEnoughSame) &&
-                wait_for_uses(pool, mem)))) {
-    *p = first->ptr;
-    pool.kept_bytes -= first->bytes;
-    pool.kept.erase(first);
-    mem.live[*p] = {want, dev};
-    return SB_OK;
-  }
-  e = cudaMalloc(p, want);
-  if (e == cudaErrorMemoryAllocation && pool.kept_bytes) {
-    cudaGetLastError();
-    trim(pool, 0, 0);
-    e = cudaMalloc(p, want);
-  }
-  if (e != cudaSuccess) {
-    *p = nullptr;
-    return cuda_status(e, "cudaMalloc");
-  }
-  mem.live[*p] = {want, dev};
-  return SB_OK;
+  const int r = current_device(&dev);
+  if (r) return r;
+  const cudaError_t e = memory().alloc(p, bytes, dev);
+  return e == cudaSuccess ? SB_OK : cuda_status(e, "cudaMalloc");
 }
 
 int device_free(void* p) {
   if (!p) return SB_OK;
-  Memory& mem = memory();
-  std::lock_guard<std::mutex> lk(mem.mu);
-  auto it = mem.live.find(p);
-  if (it == mem.live.end()) {
-    for (const Pool& pool : mem.pools)
-      for (const Block& b : pool.kept)
-        if (b.ptr == p) return cuda_status(cudaErrorInvalidValue, "cudaFree(ptr)");
-    SB_CHECK_CUDA(cudaFree(p));
-    return SB_OK;
-  }
-  const size_t bytes = it->second.first;
-  Pool& pool = mem.pools[it->second.second];
-  mem.live.erase(it);
-  if (bytes > kKeepBytes) {
-    SB_CHECK_CUDA(cudaFree(p));
-    return SB_OK;
-  }
-  trim(pool, kKeepBytes - bytes, kKeepBlocks - 1);
-  pool.kept.push_back({p, bytes, ++mem.clock});
-  pool.kept_bytes += bytes;
-  return SB_OK;
+  bool twice = false;
+  const cudaError_t e = memory().free(p, &twice);
+  if (twice) return cuda_status(cudaErrorInvalidValue, "cudaFree(ptr)");
+  return e == cudaSuccess ? SB_OK : cuda_status(e, "cudaFree");
 }
 
 int scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
@@ -251,11 +143,8 @@ int scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
     // the kept blocks of sb_free go back first
     int dev = 0;
     cudaGetLastError();
-    Memory& mem = memory();
-    std::lock_guard<std::mutex> lk(mem.mu);
-    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 &&
-        mem.pools[dev].kept_bytes) {
-      trim(mem.pools[dev], 0, 0);
+    if (current_device(&dev) == SB_OK) {
+      memory().give_back(dev, 0, 0);
       e = cudaMallocAsync(p, bytes, s);
     }
   }
@@ -477,10 +366,7 @@ int sb_mem_info(size_t* free_bytes, size_t* total_bytes) {
   if (r) return r;
   SB_CHECK_CUDA(cudaMemGetInfo(free_bytes, total_bytes));
   int dev = 0;
-  Memory& mem = memory();
-  std::lock_guard<std::mutex> lk(mem.mu);
-  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64)
-    *free_bytes += mem.pools[dev].kept_bytes;
+  if (current_device(&dev) == SB_OK) *free_bytes += memory().kept_bytes(dev);
   return SB_OK;
 }
 
