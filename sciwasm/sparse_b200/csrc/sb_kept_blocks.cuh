@@ -153,8 +153,11 @@ class KeptBlocks {
   }
 
   // Sizes are rounded so that nearly equal requests share a block: up by at most
-  // 1/64, to a multiple of 512 bytes, and by less than 2 MiB (a page).
+  // 1/64, to a multiple of 512 bytes, and by less than 2 MiB (a page).  No
+  // device has 2^62 bytes, and the last sizes would round up past zero: the
+  // driver refuses those as they are.
   static size_t round_size(size_t b) {
+    if (b >> 62) return b;
     size_t step = 512;
     while (step < (2u << 20) && step * 128 <= b) step <<= 1;
     return (b + step - 1) / step * step;

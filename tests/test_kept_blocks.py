@@ -122,6 +122,10 @@ int main() {
   // larger than all that is kept: freed at once
   put(k, get(k, 5000 * MIB));
   CHECK(k.kept_bytes(0) == 2048 * 512);
+  // sizes that would round up past zero are refused, not granted as nothing
+  Fake::room = size_t(1) << 40;
+  CHECK(k.alloc(&none, ~size_t(0), 0) == 2 && k.alloc(&none, ~size_t(0) - MIB, 0) == 2);
+  CHECK(Kept::round_size(100 * MIB + 1) == 101 * MIB && Kept::round_size(1) == 512);
   // not from here
   CHECK(Fake::malloc(&none, 64) == 0 && k.free(none, &twice) == 0 && !twice);
   std::puts("ok");
