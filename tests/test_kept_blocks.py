@@ -23,7 +23,7 @@ struct Fake {
   static inline std::set<void*> live;
   static inline uintptr_t next = 0x10000;
   static inline size_t used = 0, room = ~size_t(0);
-  static inline int mallocs = 0, frees = 0, refuse = 0;
+  static inline int mallocs = 0, frees = 0, refuse = 0, waits = 0, beside = 0;
   static inline thread_local bool held_up = false;  // this thread's frees wait for `go`
   static inline std::atomic<int> waiting{0};
   static inline std::promise<void> go;
@@ -47,6 +47,10 @@ struct Fake {
     std::lock_guard<std::mutex> lk(mu);
     if (refuse > 0) { --refuse; return 9; }
     if (!live.erase(p)) return 1;
+    if (sizes[p] == 16) {  // the waits: cheap only beside another small block
+      for (void* q : live) beside += sizes[q] == 16;
+      ++waits;
+    }
     used -= sizes[p];
     ++frees;
     return 0;
@@ -94,6 +98,7 @@ int main() {
   Fake::go.set_value();
   t.join();
   CHECK(got.get_future().get() == p[0]);
+  CHECK(Fake::waits == 1 && Fake::beside == 1);
   f = Fake::frees;
   for (int i = 1; i < 17; ++i) CHECK(get(k, MIB) == p[i]);
   CHECK(Fake::frees == f && get(k, MIB) != fresh && k.kept_bytes(0) == MIB);
