@@ -76,6 +76,10 @@ int sb_stream_create_priority(void** stream, int priority);
 int sb_stream_priority_range(int* least, int* greatest);
 int sb_stream_synchronize(void* stream);
 int sb_mem_info(size_t* free_bytes, size_t* total_bytes);
+/* Gives blocks kept by sb_free back to the driver, the oldest first, until at
+ * most keep_bytes of the current device's memory are kept (0: none): before
+ * another allocator of the process, or another process, needs the memory. */
+int sb_mem_trim(size_t keep_bytes);
 /* CUDA events for stream-ordered completion tracking and timing
  * (sb_event_query returns 1 when complete, 0 when not yet, < 0 on error). */
 int sb_event_create(void** event);

@@ -59,6 +59,7 @@ SIGNATURES: dict[str, list] = {
     "sb_stream_destroy": [P],
     "sb_stream_synchronize": [P],
     "sb_mem_info": [C.POINTER(SZ), C.POINTER(SZ)],
+    "sb_mem_trim": [SZ],
     "sb_device_status": [C.POINTER(C.c_int)],
     "sb_event_create": [C.POINTER(P)],
     "sb_event_destroy": [P],

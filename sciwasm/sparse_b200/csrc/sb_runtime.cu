@@ -208,6 +208,15 @@ int sb_malloc(void** ptr, size_t bytes) {
 
 int sb_free(void* ptr) { return device_free(ptr); }
 
+int sb_mem_trim(size_t keep_bytes) {
+  int r = ensure_device();
+  if (r) return r;
+  int dev = 0;
+  if ((r = current_device(&dev))) return r;
+  const cudaError_t e = memory().give_back(dev, keep_bytes, SIZE_MAX);
+  return e == cudaSuccess ? SB_OK : cuda_status(e, "cudaFree");
+}
+
 int sb_host_alloc(void** ptr, size_t bytes) {
   SB_REQUIRE(ptr, "sb_host_alloc: null output");
   *ptr = nullptr;

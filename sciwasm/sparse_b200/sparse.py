@@ -550,6 +550,13 @@ def free(obj) -> None:
             arr.free()
 
 
+def mem_trim(keep_bytes=0) -> None:
+    """Gives device memory that is kept for reuse after free() back to the
+    driver, down to `keep_bytes`: for other allocators (torch in the same
+    process, another process), which cannot reach it themselves."""
+    _lib.call("sb_mem_trim", int(keep_bytes))
+
+
 # --------------------------------------------------------------- SpMV
 
 

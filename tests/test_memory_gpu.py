@@ -154,3 +154,23 @@ def test_refused_allocation_is_reported_once(gpu):
     assert _lib.load().sb_malloc(ctypes.byref(q), total * 2) == _lib.SB_ENOMEM
     A = gpu.csr_from_host(np.array([0, 1, 2]), np.array([0, 1]), np.array([0.0, 3.0]))
     assert gpu.eliminate_zeros(A).nnz == 1
+
+
+def test_trim_and_bound_as_the_driver_sees_them(gpu):
+    """sb_mem_info adds kept bytes to the free ones; here the driver's own figure
+    shows how much is kept: 4 GiB at most, and what mem_trim leaves."""
+    torch = pytest.importorskip("torch")
+    raw = lambda: torch.cuda.mem_get_info()[0]
+    gpu.mem_trim()
+    free0 = raw()
+    ps = [_alloc(512 * MIB) for _ in range(10)]
+    assert free0 - raw() >= 10 * 512 * MIB
+    for p in ps:
+        _lib.call("sb_free", p)
+    slack = 64 * MIB
+    assert abs(free0 - raw() - 4096 * MIB) <= slack
+    gpu.mem_trim(1024 * MIB)
+    assert abs(free0 - raw() - 1024 * MIB) <= slack
+    assert abs(_info()[0] - raw() - 1024 * MIB) <= slack
+    gpu.mem_trim()
+    assert abs(free0 - raw()) <= slack and abs(_info()[0] - raw()) <= slack
