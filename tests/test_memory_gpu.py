@@ -174,3 +174,39 @@ def test_trim_and_bound_as_the_driver_sees_them(gpu):
     assert abs(_info()[0] - raw() - 1024 * MIB) <= slack
     gpu.mem_trim()
     assert abs(free0 - raw()) <= slack and abs(_info()[0] - raw()) <= slack
+
+
+def test_block_in_use_is_handed_out_after_a_wait(gpu):
+    """The kept block that an allocation gets is the one freed while copies out
+    of it were queued, and by then they are over: little enough is freed that no
+    block goes back to the driver, whose free would wait as well."""
+    torch = pytest.importorskip("torch")
+    n = 64 * MIB
+    gpu.mem_trim()
+    streams = []
+    for _ in range(2):
+        s = ctypes.c_void_p()
+        _lib.call("sb_stream_create", ctypes.byref(s))
+        streams.append(s.value)
+    chain = torch.cuda.ExternalStream(streams[0])
+    src, dst = _alloc(n), _alloc(n)
+    others = [_alloc(n) for _ in range(16)]
+    _lib.call("sb_memset", src, 0x5A, n, streams[0])
+    _lib.call("sb_stream_synchronize", streams[0])
+    for _ in range(500):
+        _lib.call("sb_memcpy_dtod", dst, src, n, streams[0])
+    for p in [src] + others:
+        _lib.call("sb_free", p)
+    assert not chain.query()  # sb_free has not waited
+    got = _alloc(n)
+    assert got == src and chain.query()
+    _lib.call("sb_memset", got, 0, n, streams[1])
+    _lib.call("sb_stream_synchronize", streams[1])
+    out = np.empty(n, np.uint8)
+    _lib.call("sb_memcpy_dtoh", out.ctypes.data, dst, n, None)
+    _lib.call("sb_stream_synchronize", None)
+    assert np.all(out == 0x5A)
+    for p in (got, dst):
+        _lib.call("sb_free", p)
+    for s in streams:
+        _lib.call("sb_stream_destroy", s)
