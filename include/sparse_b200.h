@@ -55,10 +55,15 @@ const char* sb_status_string(int status);
 int sb_device_count(int* count);
 int sb_set_device(int device);
 /* Device memory of the current device.  sb_free may be called while work that
- * uses the block is in flight and does not wait for it: freed blocks are kept
- * (up to 2 GiB per device) and handed out again only after a device
- * synchronisation; they go back to the driver when an allocation fails, and
- * sb_mem_info counts them as free. */
+ * uses the block is in flight: freed blocks are kept, up to 4 GiB and 2048
+ * blocks per device, and a block is handed out again only after that work is
+ * over (sb_malloc waits for the device's work where it reuses a block that has
+ * not been waited for).  sb_free itself waits, as cudaFree does, where it gives
+ * memory back to the driver: the oldest blocks beyond the bound, a block of more
+ * than 4 GiB, a pointer that is not from sb_malloc.  All kept blocks go back when
+ * an allocation of this library fails, before it is tried once more;
+ * sb_mem_info counts them as free.  Other allocators cannot reach them: see
+ * sb_mem_trim. */
 int sb_malloc(void** ptr, size_t bytes);
 int sb_free(void* ptr);
 int sb_host_alloc(void** ptr, size_t bytes); /* pinned host memory */
@@ -318,8 +323,12 @@ int sb_batch_exec_destroy(sb_batch_exec* exec);
 int sb_batch_exec_run(sb_batch_exec* exec, const sb_batch_item* items, int32_t n, void* stream);
 
 /* ---------------------------------------------------------------------- */
-/* Format conversions (bit-exact with the reference).  These calls return */
-/* after the device work is complete (they may read results to the host). */
+/* Format conversions (bit-exact with the reference).  The results are    */
+/* complete in stream order: for later work on `stream`, or after waiting */
+/* for it.  A call that returns a number has waited; the others may (all  */
+/* but sb_csr_ell read counts to the host, so only it can be captured),   */
+/* and return with their last kernels in flight or not, as the data has   */
+/* it.                                                                    */
 /* CSR inputs must have monotone row_ptr with row_ptr[0] = 0 and columns  */
 /* in [0, N); COO indices are checked on the device (SB_EINVAL).          */
 /* ---------------------------------------------------------------------- */
