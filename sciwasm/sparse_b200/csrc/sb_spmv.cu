@@ -366,9 +366,10 @@ __global__ void __launch_bounds__(256, Out::template min_blocks<T>())
   constexpr int PASS = V * UNROLL;         // entries of one unrolled pass
   // A short row needs one pass, or two where a second pass measured faster than
   // the whole-warp tail (power-law 2M FP64, V = 8: 248 -> 232 us, V = 4: 270 ->
-  // 238; but V = 8 with f32 sums 201 -> 211, V = 2 on the banded 4M FP64 matrix
-  // 124 -> 129, V = 1 on the 4096^2 Laplacian 166 -> 176)
-  constexpr int PASSES = (V == 4 || (V == 8 && sizeof(T) == 8)) ? 2 : 1;
+  // 238; but V = 2 on the banded 4M FP64 matrix 124 -> 129, V = 1 on the 4096^2
+  // Laplacian 166 -> 176).  Never for f32 sums, which the tail compensates: what
+  // is compensated doesn't depend on how fast a second pass would be.
+  constexpr int PASSES = sizeof(T) == 8 && (V == 4 || V == 8) ? 2 : 1;
   constexpr int SHORT = PASSES * PASS;
   constexpr bool COMP = sizeof(T) == 4;    // compensate long f32 sums
   const int lane = threadIdx.x & (kWarp - 1);
