@@ -390,7 +390,10 @@ __global__ void __launch_bounds__(256, Out::template min_blocks<T>())
       const int s = __shfl_sync(kFull, s_l, j);
       const int e = __shfl_sync(kFull, e_l, j);
       const int len = e - s;
-      T sum = 0;
+      // Eight entries of a lane go to two sums, so that no chain of additions is
+      // longer than with twice the lanes and half the unroll, and the sums are
+      // the same bit for bit.
+      T sum = 0, odd = 0;
       auto pass = [&](int k0) {
         int cc[UNROLL];
         T vv[UNROLL];
@@ -403,7 +406,8 @@ __global__ void __launch_bounds__(256, Out::template min_blocks<T>())
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u) {
           const int k = k0 + u * V;
-          if (k < e) sum += vv[u] * ld_ro(x + cc[u]);
+          T& acc = UNROLL == 8 && (u & 1) ? odd : sum;
+          if (k < e) acc += vv[u] * ld_ro(x + cc[u]);
         }
       };
       if constexpr (PASSES == 1) {
@@ -412,6 +416,7 @@ __global__ void __launch_bounds__(256, Out::template min_blocks<T>())
         for (int k0 = s + q; __any_sync(kFull, k0 < e && len <= SHORT); k0 += PASS)
           if (len <= SHORT) pass(k0);
       }
+      if (UNROLL == 8) sum += odd;
 #pragma unroll
       for (int off = V >> 1; off > 0; off >>= 1) sum += __shfl_xor_sync(kFull, sum, off);
       const T yj = __shfl_sync(kFull, y_l, j);

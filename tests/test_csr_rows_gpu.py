@@ -55,3 +55,32 @@ def test_edges_of_passes(gpu, dt, lanes, unroll, grid):
         else:
             tol = n * u * mass
         assert abs(y[i] - want) <= tol, (i, n, y[i], want, tol)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("kind", ["five", "boundary", "eleven", "poisson4", "poisson10", "mixed4",
+                                  "mixed10", "empty"])
+def test_default_sums_of_short_rows(gpu, dt, kind):
+    """Without options, rows of up to one pass are summed as two lanes (four for
+    means above 6) with four entries each sum them, bit for bit."""
+    rng = np.random.default_rng(5)
+    N = 32 * 70 + 13
+    lens = {"five": np.full(N, 5), "boundary": np.where(np.arange(N) % 37, 7, 6),
+            "eleven": np.full(N, 11), "poisson4": rng.poisson(4, N), "poisson10": rng.poisson(10, N),
+            "mixed4": np.where(np.arange(N) // 32 % 2, 4, rng.poisson(4, N)),
+            "mixed10": np.where(np.arange(N) // 32 % 2, 9, rng.poisson(10, N)),
+            "empty": np.where(rng.random(N) < 0.9, 0, 8)}[kind]
+    lanes = 2 if lens.mean() <= 6 else 4
+    if dt == np.float64:
+        lens = np.minimum(lens, 4 * lanes)  # (four lanes take two passes in FP64)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    col = rng.integers(0, N, rp[-1]).astype(np.int32)
+    A = gpu.csr_from_host(rp, col, rng.standard_normal(rp[-1]).astype(dt))
+    x, y0 = gpu.vec_from_host(rng.standard_normal(N).astype(dt)), rng.standard_normal(N).astype(dt)
+    ys = []
+    for opts in (None, _lib.CsrOpts(0, lanes, 4, 0)):
+        A.opts = opts
+        yv = gpu.vec_from_host(y0)
+        gpu.spmv(A, x, yv)
+        ys.append(yv.array())
+    assert np.array_equal(ys[0].view(np.uint8), ys[1].view(np.uint8))
