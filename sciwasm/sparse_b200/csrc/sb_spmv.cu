@@ -296,6 +296,49 @@ __device__ __forceinline__ float ld_val(const __nv_bfloat16* p) {
   return __bfloat162float(__ushort_as_bfloat16(ld_stream(reinterpret_cast<const unsigned short*>(p))));
 }
 
+// *p where `on`, else 0, as one predicated load.  Written as a condition in C++,
+// the loads of an unrolled group become branches around each entry's chain of
+// index, value and x wherever the compiler sees fit, which varies from one
+// instance of the row kernel to the next.  The kernel takes ld_if for the
+// whole-warp tail and for short rows of 4 lanes and more, but conditions where
+// those measured faster: V <= 2 (5-point Laplacian of 4M rows bf16, V = 1, 39 us
+// and 50; its tail too, FP64 58 and 61), FP64 with V >= 16 (4M rows of
+// Poisson(40) entries, random columns, 744 and 783), and stores to several
+// arrays, whose 32 registers would spill.  Measured on B200 (us, conditions
+// everywhere -> now): rows of 5 + Zipf(2) entries, 1M of them, f32 92 -> 74, FP64
+// 101 -> 83; of 15 + Zipf(2), 4M, 367 -> 359 and 423 -> 404; 41 diagonals of 1M rows
+// f32 112 -> 72; 27-point stencil of 4M rows f32 184 -> 171, FP64 273 -> 261; 15
+// diagonals FP64 206 -> 183.  What lost: 7-point stencil FP64 77 -> 80, 9-point
+// 89 -> 92.
+__device__ __forceinline__ int ld_if(const int* p, bool on) {
+  int v;
+  asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %2, 0;\nmov.b32 %0, 0;\n"
+               "@q ld.global.nc.b32 %0, [%1];\n}"
+               : "=r"(v) : "l"(p), "r"((int)on));
+  return v;
+}
+__device__ __forceinline__ float ld_if(const float* p, bool on) {
+  float v;
+  asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %2, 0;\nmov.f32 %0, 0f00000000;\n"
+               "@q ld.global.nc.f32 %0, [%1];\n}"
+               : "=f"(v) : "l"(p), "r"((int)on));
+  return v;
+}
+__device__ __forceinline__ double ld_if(const double* p, bool on) {
+  double v;
+  asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %2, 0;\nmov.f64 %0, 0d0000000000000000;\n"
+               "@q ld.global.nc.f64 %0, [%1];\n}"
+               : "=d"(v) : "l"(p), "r"((int)on));
+  return v;
+}
+__device__ __forceinline__ float ld_if(const __nv_bfloat16* p, bool on) {
+  unsigned short v;
+  asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %2, 0;\nmov.b16 %0, 0;\n"
+               "@q ld.global.nc.b16 %0, [%1];\n}"
+               : "=h"(v) : "l"(p), "r"((int)on));
+  return __bfloat162float(__ushort_as_bfloat16(v));
+}
+
 // Neumaier-compensated accumulation (used for long rows with f32 sums).
 template <typename T>
 __device__ __forceinline__ void comp_add(T& s, T& c, T v) {
@@ -357,24 +400,81 @@ struct YScatter {
   }
 };
 
+// The rows of a block of 32 with at most SHORT entries, in batches of 32/V rows
+// with V lanes each; TWO: rows may take two passes of V * UNROLL entries.
+template <typename SV, typename T, int V, int UNROLL, bool TWO, int SHORT, class Out>
+__device__ __forceinline__ void csr_short_rows(const int* __restrict__ col,
+                                               const SV* __restrict__ val,
+                                               const T* __restrict__ x, const Out& out, int N,
+                                               int r0, int s_l, int e_l, T y_l) {
+  constexpr int RPB = kWarp / V;     // rows per batch
+  constexpr int PASS = V * UNROLL;   // entries of one unrolled pass
+  constexpr bool PRED = !Out::kAll && (sizeof(T) == 4 ? V > 2 : V == 4 || V == 8);  // see ld_if
+  const int lane = threadIdx.x & (kWarp - 1);
+  const int g = lane / V;
+  const int q = lane - g * V;
+#pragma unroll
+  for (int b = 0; b < V; ++b) {
+    const int j = b * RPB + g;  // row of this group within the block
+    const int s = __shfl_sync(kFull, s_l, j);
+    const int e = __shfl_sync(kFull, e_l, j);
+    const int len = e - s;
+    // Eight entries of a lane go to two sums, so that no chain of additions is
+    // longer than with twice the lanes and half the unroll, and the sums are
+    // the same bit for bit.
+    T sum = 0, odd = 0;
+    auto pass = [&](int k0) {
+      int cc[UNROLL];
+      T vv[UNROLL];
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u) {
+        const int k = k0 + u * V;
+        if constexpr (!PRED) {
+          cc[u] = k < e ? ld_reuse(col + k) : 0;
+          vv[u] = k < e ? (T)ld_val_reuse(val + k) : (T)0;
+        } else {
+          cc[u] = ld_if(col + k, k < e);
+          vv[u] = (T)ld_if(val + k, k < e);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < UNROLL; ++u) {
+        const int k = k0 + u * V;
+        T& acc = UNROLL == 8 && (u & 1) ? odd : sum;
+        if (k < e) acc += vv[u] * ld_ro(x + cc[u]);
+      }
+    };
+    if constexpr (!TWO) {
+      if (len <= SHORT) pass(s + q);
+    } else {
+      for (int k0 = s + q; __any_sync(kFull, k0 < e && len <= SHORT); k0 += PASS)
+        if (len <= SHORT) pass(k0);
+    }
+    if (UNROLL == 8) sum += odd;
+#pragma unroll
+    for (int off = V >> 1; off > 0; off >>= 1) sum += __shfl_xor_sync(kFull, sum, off);
+    const T yj = __shfl_sync(kFull, y_l, j);
+    if (q == 0 && len > 0 && len <= SHORT && r0 + j < N) out.put(r0 + j, yj + sum);
+    else if (Out::kAll && q == 0 && len == 0 && r0 + j < N) out.put(r0 + j, yj);
+  }
+}
+
 template <typename SV, typename T, int V, int UNROLL, class Out>
 __global__ void __launch_bounds__(256, Out::template min_blocks<T>())
     csr_rows_kernel(const int* __restrict__ row_ptr, const int* __restrict__ col,
                     const SV* __restrict__ val, const T* __restrict__ x, const T* y_in,
                     Out out, int N) {
-  constexpr int RPB = kWarp / V;           // rows per batch
-  constexpr int PASS = V * UNROLL;         // entries of one unrolled pass
+  constexpr int PASS = V * UNROLL;
   // A short row needs one pass, or two where a second pass measured faster than
   // the whole-warp tail (power-law 2M FP64, V = 8: 248 -> 232 us, V = 4: 270 ->
   // 238; but V = 2 on the banded 4M FP64 matrix 124 -> 129, V = 1 on the 4096^2
   // Laplacian 166 -> 176).  Never for f32 sums, which the tail compensates: what
-  // is compensated doesn't depend on how fast a second pass would be.
+  // is compensated doesn't depend on how fast a second pass would be.  Blocks
+  // without a row of two passes go without its loop.
   constexpr int PASSES = sizeof(T) == 8 && (V == 4 || V == 8) ? 2 : 1;
   constexpr int SHORT = PASSES * PASS;
   constexpr bool COMP = sizeof(T) == 4;    // compensate long f32 sums
   const int lane = threadIdx.x & (kWarp - 1);
-  const int g = lane / V;
-  const int q = lane - g * V;
   const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
   for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
        w * kWarp < N; w += warps) {
@@ -384,44 +484,13 @@ __global__ void __launch_bounds__(256, Out::template min_blocks<T>())
     const int e_l = rr < N ? __ldg(row_ptr + rr + 1) : 0;
     const int len_l = e_l - s_l;
     const T y_l = (rr < N && (len_l > 0 || Out::kAll)) ? y_in[rr] : (T)0;
-#pragma unroll
-    for (int b = 0; b < V; ++b) {
-      const int j = b * RPB + g;  // row of this group within the block
-      const int s = __shfl_sync(kFull, s_l, j);
-      const int e = __shfl_sync(kFull, e_l, j);
-      const int len = e - s;
-      // Eight entries of a lane go to two sums, so that no chain of additions is
-      // longer than with twice the lanes and half the unroll, and the sums are
-      // the same bit for bit.
-      T sum = 0, odd = 0;
-      auto pass = [&](int k0) {
-        int cc[UNROLL];
-        T vv[UNROLL];
-#pragma unroll
-        for (int u = 0; u < UNROLL; ++u) {
-          const int k = k0 + u * V;
-          cc[u] = k < e ? ld_reuse(col + k) : 0;
-          vv[u] = k < e ? (T)ld_val_reuse(val + k) : (T)0;
-        }
-#pragma unroll
-        for (int u = 0; u < UNROLL; ++u) {
-          const int k = k0 + u * V;
-          T& acc = UNROLL == 8 && (u & 1) ? odd : sum;
-          if (k < e) acc += vv[u] * ld_ro(x + cc[u]);
-        }
-      };
-      if constexpr (PASSES == 1) {
-        if (len <= SHORT) pass(s + q);
-      } else {
-        for (int k0 = s + q; __any_sync(kFull, k0 < e && len <= SHORT); k0 += PASS)
-          if (len <= SHORT) pass(k0);
-      }
-      if (UNROLL == 8) sum += odd;
-#pragma unroll
-      for (int off = V >> 1; off > 0; off >>= 1) sum += __shfl_xor_sync(kFull, sum, off);
-      const T yj = __shfl_sync(kFull, y_l, j);
-      if (q == 0 && len > 0 && len <= SHORT && r0 + j < N) out.put(r0 + j, yj + sum);
-      else if (Out::kAll && q == 0 && len == 0 && r0 + j < N) out.put(r0 + j, yj);
+    if constexpr (PASSES == 2) {
+      if (__any_sync(kFull, len_l > PASS && len_l <= SHORT))
+        csr_short_rows<SV, T, V, UNROLL, true, SHORT>(col, val, x, out, N, r0, s_l, e_l, y_l);
+      else
+        csr_short_rows<SV, T, V, UNROLL, false, SHORT>(col, val, x, out, N, r0, s_l, e_l, y_l);
+    } else {
+      csr_short_rows<SV, T, V, UNROLL, false, SHORT>(col, val, x, out, N, r0, s_l, e_l, y_l);
     }
     // long rows of the block: whole warp each
     unsigned longm = __ballot_sync(kFull, rr < N && len_l > SHORT);
@@ -437,8 +506,13 @@ __global__ void __launch_bounds__(256, Out::template min_blocks<T>())
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int k = k0 + lane + u * kWarp;
-          cc[u] = k < e ? ld_reuse(col + k) : 0;
-          vv[u] = k < e ? (T)ld_val_reuse(val + k) : (T)0;
+          if constexpr (V == 1 || Out::kAll) {
+            cc[u] = k < e ? ld_reuse(col + k) : 0;
+            vv[u] = k < e ? (T)ld_val_reuse(val + k) : (T)0;
+          } else {
+            cc[u] = ld_if(col + k, k < e);
+            vv[u] = (T)ld_if(val + k, k < e);
+          }
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -504,28 +578,33 @@ static int default_lanes(int N, long long nnz) {
   return 16;
 }
 
-// Options of a call that gives none, from the mean row length.  Few lanes with
-// a long unroll for short rows: a lane's loads of consecutive entries share
-// sectors, and no shuffle follows.  One warp per block of rows for longer ones,
-// whose lengths usually differ.  Measured on B200 (us, with the lanes above,
-// unroll 4 and the resident grid -> now): Laplacian 4096^2 FP32 199 -> 166, FP64
-// 252 -> 234; banded 4M x 11 FP64 125 -> 119, FP32 98 -> 86; power-law 2M FP64
-// 256 -> 232, FP32 225 -> 199; rows of Poisson(5) entries, random columns, 1M
-// rows FP32 43 -> 41, FP64 43 -> 45.
-static sb_csr_opts default_opts(int N, long long nnz) {
-  const double avg = N ? (double)nnz / N : 0.0;
-  if (avg <= 6) return {0, 1, 8, 0};
-  if (avg <= 14) return {0, 2, 8, 0};
-  if (avg <= 28) return {0, 8, 4, 1};
-  return {0, 16, 4, 1};
-}
-
+// opts: null for a call that gives none.  Its launch then follows the mean row
+// length: few lanes with a long unroll for short rows, as a lane's loads of
+// consecutive entries share sectors, and few or no shuffles follow.  One warp
+// per block of rows for longer ones, whose lengths usually differ.  Measured on
+// B200 against 2 / 4 / 8 / 16 lanes (means to 6 / 14 / 28 / more) with unroll 4 and
+// the resident grid, 4M rows, us, those -> now, f32 and FP64:
+//   5-point Laplacian        50 -> 43    64 -> 58
+//   11 diagonals             87 -> 73   114 -> 110
+//   27-point stencil        184 -> 171  258 -> 261
+//   15 diagonals            150 -> 123  164 -> 183
+//   Poisson(10), random     193 -> 191  218 -> 220
+//   Poisson(20), random     370 -> 331  408 -> 365
+//   Poisson(40), random     742 -> 656  757 -> 745
+//   15 + Zipf(2), random    424 -> 359  464 -> 404
+// The mean can't tell 15 equal FP64 entries from 15 unequal ones, which gain.
 template <typename SV, typename T, class Out>
 static int launch_csr_rows_out(const int* row_ptr, const int* col, const SV* val, const T* x,
-                               const T* y_in, Out out, int N, long long nnz, int lanes,
-                               int unroll, int grid, cudaStream_t st) {
-  if (lanes <= 0) lanes = default_lanes(N, nnz);
-  if (unroll <= 0) unroll = 4;
+                               const T* y_in, Out out, int N, long long nnz,
+                               const sb_csr_opts* opts, cudaStream_t st) {
+  const double avg = N ? (double)nnz / N : 0.0;
+  if (!opts && avg <= 14) {
+    if (avg <= 6)
+      return launch_csr_rows_v<SV, T, 1, 8>(row_ptr, col, val, x, y_in, out, N, 0, st);
+    return launch_csr_rows_v<SV, T, 2, 8>(row_ptr, col, val, x, y_in, out, N, 0, st);
+  }
+  const int lanes = opts && opts->lanes_per_row > 0 ? opts->lanes_per_row : default_lanes(N, nnz);
+  const int unroll = opts && opts->unroll > 0 ? opts->unroll : 4, grid = opts ? opts->grid : 1;
 #define SB_CSR_L(v) \
   return launch_csr_rows_u<SV, T, v>(row_ptr, col, val, x, y_in, out, N, unroll, grid, st)
   switch (lanes) {
@@ -541,10 +620,8 @@ static int launch_csr_rows_out(const int* row_ptr, const int* col, const SV* val
 
 template <typename SV, typename T>
 static int launch_csr_rows(const int* row_ptr, const int* col, const SV* val, const T* x, T* y,
-                           int N, long long nnz, int lanes, int unroll, int grid,
-                           cudaStream_t st) {
-  return launch_csr_rows_out<SV, T>(row_ptr, col, val, x, y, YOut<T>{y}, N, nnz, lanes, unroll,
-                                    grid, st);
+                           int N, long long nnz, const sb_csr_opts* opts, cudaStream_t st) {
+  return launch_csr_rows_out<SV, T>(row_ptr, col, val, x, y, YOut<T>{y}, N, nnz, opts, st);
 }
 
 // ------------------------------------------------------------ COO
@@ -1522,9 +1599,7 @@ static int launch_csr(const int* row_ptr, const int* col, const S* val, const S*
     if (opts->unroll == 2048) return launch_csr_stream<S, 2048, 3>(row_ptr, col, val, x, y, N, nnz, st);
     return launch_csr_stream<S, 1024, 4>(row_ptr, col, val, x, y, N, nnz, st);
   }
-  const sb_csr_opts o = opts ? *opts : default_opts(N, nnz);
-  return launch_csr_rows<S, S>(row_ptr, col, val, x, y, N, nnz, o.lanes_per_row, o.unroll, o.grid,
-                               st);
+  return launch_csr_rows<S, S>(row_ptr, col, val, x, y, N, nnz, opts, st);
 }
 
 template <typename S, typename A>
@@ -1584,8 +1659,6 @@ int sb_spmv_csr_allgather(int dtype, const int32_t* row_ptr, const int32_t* col,
   int r = ensure_device();
   if (r) return r;
   cudaStream_t st = as_stream(stream);
-  const sb_csr_opts o = opts ? *opts : default_opts(rows, nnz);
-  const int lanes = o.lanes_per_row, unroll = o.unroll, grid = o.grid;
   const unsigned long long* dd = reinterpret_cast<const unsigned long long*>(dst);
   if (dtype == SB_F64) {
     YScatter<double> out{};
@@ -1594,7 +1667,7 @@ int sb_spmv_csr_allgather(int dtype, const int32_t* row_ptr, const int32_t* col,
     out.r0 = row_offset;
     return launch_csr_rows_out<double, double>(row_ptr, col, (const double*)val,
                                                (const double*)x, (const double*)y_in, out, rows,
-                                               nnz, lanes, unroll, grid, st);
+                                               nnz, opts, st);
   }
   YScatter<float> out{};
   out.d = dd;
@@ -1603,10 +1676,9 @@ int sb_spmv_csr_allgather(int dtype, const int32_t* row_ptr, const int32_t* col,
   if (dtype == SB_BF16)
     return launch_csr_rows_out<__nv_bfloat16, float>(row_ptr, col, (const __nv_bfloat16*)val,
                                                      (const float*)x, (const float*)y_in, out,
-                                                     rows, nnz, lanes, unroll, grid, st);
+                                                     rows, nnz, opts, st);
   return launch_csr_rows_out<float, float>(row_ptr, col, (const float*)val, (const float*)x,
-                                           (const float*)y_in, out, rows, nnz, lanes, unroll,
-                                           grid, st);
+                                           (const float*)y_in, out, rows, nnz, opts, st);
 }
 
 int sb_spmv_csr_ex(int dtype, const int32_t* row_ptr, const int32_t* col, const void* val,
@@ -1637,12 +1709,9 @@ int sb_spmv_csr_ex(int dtype, const int32_t* row_ptr, const int32_t* col, const 
     else if (dtype == SB_BF16 && opts && opts->kernel == 3)
       r = launch_csr_block_stream<__nv_bfloat16, float>(row_ptr, col, (const __nv_bfloat16*)val,
                                                         (const float*)x, (float*)y, N, nnz, st);
-    else if (dtype == SB_BF16) {
-      const sb_csr_opts o = opts ? *opts : default_opts(N, nnz);
+    else if (dtype == SB_BF16)
       r = launch_csr_rows<__nv_bfloat16, float>(row_ptr, col, (const __nv_bfloat16*)val,
-                                                (const float*)x, (float*)y, N, nnz,
-                                                o.lanes_per_row, o.unroll, o.grid, st);
-    }
+                                                (const float*)x, (float*)y, N, nnz, opts, st);
     else if (dtype == SB_F32)
       r = launch_csr<float, float>(row_ptr, col, (const float*)val, (const float*)x, (float*)y, N,
                                    nnz, opts, st);
