@@ -69,11 +69,45 @@ __device__ __forceinline__ int bucket_add(int* cnt, int b, bool on) {
   return base + __popc(peers & ((1u << lane) - 1u));
 }
 
-// Bucket sizes; flags[0] = 1: an index out of range (with `check`; columns
-// where they are given).
+// What the passes below leave for the host.
+struct Flags {
+  int bad;       // an index out of range
+  int largest;   // bucket
+  int listed[2]; // buckets for the medium and the large sort
+  int unfit;     // the sample found a row beyond a bucket
+  int slots;     // buckets beyond the large sort
+  int runs[kMaxShift + 1];  // their largest run of 2^s rows
+};
+
+// One row beyond kLarge entries makes the buckets useless, and where it holds a
+// good part of the entries, counting them costs more than all else, since its
+// atomics queue up on one address.  A sample of kSamples entries, counted by
+// rows in a hashed table, finds such a row before the count (a shuffled row of
+// 4M among 18M entries: transpose 5.7 -> 1.6 ms on B200, the radix sort included;
+// columns with a density of 1/c 6.9 -> 1.6, as rows of coo_csr 9.6 -> 2.5; 5 us for
+// matrices without one).  `least` sightings stand for more than
+// kLarge entries; a row that is missed, or met by chance, costs time only.
+constexpr int kSamples = 16384;
+constexpr long long kSampleFrom = 1 << 20;  // entries from which the sample pays
+
+__global__ void __launch_bounds__(kThreads)
+    bucket_sample(const int* __restrict__ row, long long nnz, int least, int* __restrict__ table,
+                  Flags* __restrict__ flags) {
+  const unsigned i = blockIdx.x * kThreads + threadIdx.x;
+  const long long step = nnz / kSamples;
+  const unsigned r = ld_stream(row + i * step + (i * 2654435761u >> 8) % (unsigned)step);
+  if (atomicAdd(table + (r * 2654435761u) / (unsigned)(0x100000000ull / kSamples), 1) + 1 == least)
+    flags->unfit = 1;
+}
+
+// Bucket sizes (cnt null, or a sample that found them useless: only the check);
+// flags: an index out of range (with `check`; columns where they are given).
 __global__ void __launch_bounds__(kThreads)
     bucket_count(const int* __restrict__ row, const int* __restrict__ col, long long nnz, int rows,
-                 int cols, bool check, int shift, int* __restrict__ cnt, int* __restrict__ flags) {
+                 int cols, bool check, int shift, int* __restrict__ cnt,
+                 Flags* __restrict__ flags) {
+  const bool count = cnt && !flags->unfit;
+  if (!count && !check) return;
   const long long base = (long long)blockIdx.x * kThreads * kItemsPerThread + threadIdx.x;
   int r[kItemsPerThread];
   bool bad = false;
@@ -91,24 +125,59 @@ __global__ void __launch_bounds__(kThreads)
       on = false;
       r[u] = 0;
     }
-    bucket_add(cnt, r[u] >> shift, on);
+    if (count) bucket_add(cnt, r[u] >> shift, on);
   }
-  if (bad) flags[0] = 1;
+  if (bad) flags->bad = 1;
 }
 
 // The padded counts into start[0 .. n) (to be scanned; start[n] = 0); the
-// largest into flags[1].
+// largest into flags.
 __global__ void bucket_sizes(const int* __restrict__ cnt, int n, int* __restrict__ start,
-                             int* __restrict__ flags) {
+                             Flags* __restrict__ flags) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int c = i < n ? cnt[(size_t)i * kPad] : 0;
   if (i <= n) start[i] = c;
   const int m = __reduce_max_sync(0xffffffffu, c);
-  if ((threadIdx.x & 31) == 0 && m > flags[1]) atomicMax(flags + 1, m);
+  if ((threadIdx.x & 31) == 0 && m > flags->largest) atomicMax(&flags->largest, m);
 }
 __global__ void bucket_cursors(const int* __restrict__ start, int n, int* __restrict__ cursor) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) cursor[(size_t)i * kPad] = start[i];
+}
+
+// Buckets beyond the large sort: their slots (slot[b], else -1), the entries of
+// each of their rows, and from these the largest runs of 2^s rows, which tell
+// how far the buckets have to be cut down, if that helps.
+__global__ void bucket_slots(const int* __restrict__ cnt, int n, int* __restrict__ slot,
+                             Flags* __restrict__ flags) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) slot[i] = cnt[(size_t)i * kPad] > kLarge ? atomicAdd(&flags->slots, 1) : -1;
+}
+__global__ void __launch_bounds__(kThreads)
+    bucket_rows(const int* __restrict__ row, long long nnz, int shift,
+                const int* __restrict__ slot, int* __restrict__ row_cnt) {
+  const long long base = (long long)blockIdx.x * kThreads * kItemsPerThread + threadIdx.x;
+#pragma unroll
+  for (int u = 0; u < kItemsPerThread; ++u) {
+    const long long k = base + u * kThreads;
+    if (k >= nnz) continue;
+    const int r = ld_stream(row + k), s = slot[r >> shift];
+    if (s >= 0) atomicAdd(row_cnt + ((size_t)s << shift) + (r & ((1 << shift) - 1)), 1);
+  }
+}
+__global__ void __launch_bounds__(1 << kMaxShift)
+    bucket_runs(const int* __restrict__ row_cnt, int shift, Flags* __restrict__ flags) {
+  __shared__ int sum[1 << kMaxShift];
+  const int t = threadIdx.x;
+  if ((int)blockIdx.x >= flags->slots) return;
+  sum[t] = t < 1 << shift ? row_cnt[((size_t)blockIdx.x << shift) + t] : 0;
+  for (int s = 0; s <= shift; ++s) {  // sum[i << s]: rows i << s to (i + 1) << s
+    __syncthreads();
+    const int v = t & ((1 << s) - 1) ? 0 : sum[t];
+    if (v > kLarge) atomicMax(&flags->runs[s], v);
+    __syncthreads();
+    if (s < shift && (t & ((2 << s) - 1)) == 0) sum[t] = v + sum[t + (1 << s)];
+  }
 }
 
 struct Bits {
@@ -330,84 +399,108 @@ int bucket_csr(const int* row, const int* col, const int* csr_ptr, const T* val,
   while (bits.shift < kMaxShift && ((long long)nnz << (bits.shift + 1)) <= 1024LL * rows)
     ++bits.shift;
   bits.shift = std::min(bits.shift, 63 - bits.col - bits.pos);
-  int* mem = nullptr;
+  int *mem = nullptr, *cnt = nullptr, *start = nullptr, *list = nullptr;
   Item* items = nullptr;
-  int r = SB_OK, nb = 0;
-  int *cnt = nullptr, *start = nullptr, *list = nullptr, *flags = nullptr;
-  cudaError_t e = cudaSuccess;
-  int hf[2] = {0, 0};  // an index out of range; the largest bucket
-  while (true) {
+  Flags* flags = nullptr;
+  Flags hf = {};
+  int nb = 0, r = SB_OK;
+  const bool sample = nnz >= kSampleFrom;
+  const size_t head = sizeof(Flags) + (sample ? sizeof(int) * kSamples : 0);  // and the table
+  if ((r = scratch_alloc((void**)&flags, head, st))) return r;
+  cudaError_t e = cudaMemsetAsync(flags, 0, head, st);
+  if (e == cudaSuccess && sample) {
+    const int least = std::max(24, (int)(1.25 * kLarge * kSamples / (double)nnz));
+    bucket_sample<<<kSamples / kThreads, kThreads, 0, st>>>(row, nnz, least, (int*)(flags + 1),
+                                                            flags);
+    e = cudaGetLastError();
+  }
+  for (bool cut = false; e == cudaSuccess; cut = true) {
     nb = (int)((((long long)rows - 1) >> bits.shift) + 1);
-    // cnt[nb] padded, start[nb + 1], lists[2][nb], flags[4]: out of range, largest, listed
-    const size_t ints = (size_t)nb * (kPad + 3) + 5;
-    if ((r = scratch_alloc((void**)&mem, sizeof(int) * ints, st))) return r;
+    // cnt[nb] padded, start[nb + 1], lists[2][nb]; without memory for them the
+    // entries are still checked
+    const size_t ints = (size_t)nb * (kPad + 3) + 1;
+    if (scratch_alloc((void**)&mem, sizeof(int) * ints, st)) mem = nullptr;
     cnt = mem;
     start = mem + (size_t)nb * kPad;
     list = start + nb + 1;
-    flags = list + 2 * (size_t)nb;
-    e = cudaMemsetAsync(mem, 0, sizeof(int) * (size_t)nb * kPad, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, sizeof(int) * 4, st);
+    if (mem) e = cudaMemsetAsync(mem, 0, sizeof(int) * (size_t)nb * kPad, st);
     if (e == cudaSuccess) {
       bucket_count<<<blocks_for(nnz, kThreads * kItemsPerThread), kThreads, 0, st>>>(
-          row, col, nnz, rows, cols, check, bits.shift, cnt, flags);
-      bucket_sizes<<<blocks_for((long long)nb + 1, kThreads), kThreads, 0, st>>>(cnt, nb, start,
-                                                                              flags);
+          row, col, nnz, rows, cols, check && !cut, bits.shift, cnt, flags);
+      if (mem)
+        bucket_sizes<<<blocks_for((long long)nb + 1, kThreads), kThreads, 0, st>>>(cnt, nb, start,
+                                                                                flags);
       e = cudaGetLastError();
     }
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) r = cuda_status(e, "bucket_csr (counts)");
-    if (!r && hf[0]) {
+    if (e != cudaSuccess) break;
+    if (hf.bad) {
       set_error("index outside [0, %d)", rows);
       r = SB_EINVAL;
+      break;
     }
-    if (r || hf[1] <= kLarge || bits.shift == 0) break;
-    // a bucket beyond shared memory (long rows next to one another): fewer rows
-    while (bits.shift > 0 && hf[1] > kLarge) {
-      --bits.shift;
-      hf[1] = (hf[1] + 1) / 2;
+    if (mem && !hf.unfit && hf.largest <= kLarge) break;
+    r = kBucketsUnfit;
+    if (!mem || hf.unfit || cut || bits.shift == 0) break;
+    // buckets beyond shared memory (long rows next to one another, or one row):
+    // fewer rows to a bucket, as few as it takes
+    int* row_cnt = nullptr;
+    const int most = (int)(nnz / kLarge) + 1;
+    const size_t bytes = sizeof(int) * ((size_t)most << bits.shift);
+    if (scratch_alloc((void**)&row_cnt, bytes, st)) break;
+    e = cudaMemsetAsync(row_cnt, 0, bytes, st);
+    if (e == cudaSuccess) {
+      bucket_slots<<<blocks_for(nb, kThreads), kThreads, 0, st>>>(cnt, nb, list, flags);
+      bucket_rows<<<blocks_for(nnz, kThreads * kItemsPerThread), kThreads, 0, st>>>(
+          row, nnz, bits.shift, list, row_cnt);
+      bucket_runs<<<most, 1 << kMaxShift, 0, st>>>(row_cnt, bits.shift, flags);
+      e = cudaGetLastError();
     }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, sizeof(Flags), st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    scratch_free(row_cnt, st);
+    if (e != cudaSuccess || hf.runs[0] > kLarge) break;
+    while (bits.shift > 0 && hf.runs[bits.shift] > kLarge) --bits.shift;
+    r = SB_OK;
     scratch_free(mem, st);
     mem = nullptr;
   }
-  if (!r && hf[1] > kLarge) r = kBucketsUnfit;
+  if (e != cudaSuccess) r = cuda_status(e, "bucket_csr (counts)");
   if (!r) r = prim::exclusive_scan(start, start, (long long)nb + 1, st);
-  if (!r) r = scratch_alloc((void**)&items, sizeof(Item) * (size_t)nnz, st);
+  if (!r && scratch_alloc((void**)&items, sizeof(Item) * (size_t)nnz, st)) r = kBucketsUnfit;
   if (!r) {
-    {
-      bucket_cursors<<<blocks_for(nb, kThreads), kThreads, 0, st>>>(start, nb, cnt);
-      if (csr_ptr)
-        bucket_scatter_csr<T><<<blocks_for(cols, kThreads), kThreads, 0, st>>>(
-            csr_ptr, row, val, cols, bits, cnt, items);
-      else
-        bucket_scatter<T><<<blocks_for(nnz, kThreads * kScatterItems), kThreads, 0, st>>>(row, col, val, nnz,
-                                                                              bits, cnt, items);
-      e = cudaGetLastError();
-    }
-    // flags[2], flags[3]: buckets listed for the medium and the large form
+    bucket_cursors<<<blocks_for(nb, kThreads), kThreads, 0, st>>>(start, nb, cnt);
+    if (csr_ptr)
+      bucket_scatter_csr<T><<<blocks_for(cols, kThreads), kThreads, 0, st>>>(csr_ptr, row, val,
+                                                                             cols, bits, cnt, items);
+    else
+      bucket_scatter<T><<<blocks_for(nnz, kThreads * kScatterItems), kThreads, 0, st>>>(
+          row, col, val, nnz, bits, cnt, items);
+    e = cudaGetLastError();
     auto small = bucket_sort<T, kSmall, kThreads>;
     auto medium = bucket_sort<T, kMedium, 512>;
     auto large = bucket_sort<T, kLarge, 1024>;
     if (e == cudaSuccess) {
       small<<<std::min(nb, 1 << 20), kThreads, 16 * kSmall, st>>>(
-          items, start, nb, rows, bits, nullptr, nullptr, list, flags + 2, out_ptr, out_col,
+          items, start, nb, rows, bits, nullptr, nullptr, list, flags->listed, out_ptr, out_col,
           out_val);
       e = cudaGetLastError();
     }
-    if (e == cudaSuccess && hf[1] > kSmall) {
-      medium<<<4 * sm_count(), 512, 16 * kMedium, st>>>(items, start, nb, rows, bits, list,
-                                                        flags + 2, list + nb, flags + 3, out_ptr,
-                                                        out_col, out_val);
+    if (e == cudaSuccess && hf.largest > kSmall) {
+      medium<<<4 * sm_count(), 512, 16 * kMedium, st>>>(
+          items, start, nb, rows, bits, list, flags->listed, list + nb, flags->listed + 1, out_ptr,
+          out_col, out_val);
       e = cudaGetLastError();
     }
-    if (e == cudaSuccess && hf[1] > kMedium) {
+    if (e == cudaSuccess && hf.largest > kMedium) {
       e = cudaFuncSetAttribute((const void*)large, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                16 * kLarge);
       if (e == cudaSuccess) {
         large<<<sm_count(), 1024, 16 * kLarge, st>>>(items, start, nb, rows, bits, list + nb,
-                                                     flags + 3, nullptr, nullptr, out_ptr, out_col,
-                                                     out_val);
+                                                     flags->listed + 1, nullptr, nullptr, out_ptr,
+                                                     out_col, out_val);
         e = cudaGetLastError();
       }
     }
@@ -416,6 +509,7 @@ int bucket_csr(const int* row, const int* col, const int* csr_ptr, const T* val,
   }
   if (items) scratch_free(items, st);
   if (mem) scratch_free(mem, st);
+  scratch_free(flags, st);
   return r;
 }
 

@@ -7,8 +7,9 @@
 
 namespace sb {
 
-// Returned by the bucket sort, with nothing written, when the entries do not
-// suit it (a bucket beyond shared memory, or keys of more than 64 bits).
+// Returned by the bucket sort, with nothing written but the indices checked,
+// when the entries do not suit it (a row beyond shared memory) or its scratch
+// memory cannot be had: the caller's radix sort takes over.
 constexpr int kBucketsUnfit = 1;
 
 // Entry k is (row[k], col[k], val[k]); with csr_ptr (and row) given instead of

@@ -91,3 +91,55 @@ def test_index_out_of_range_after_the_prefix(gpu, where):
     A.col_index.upload(col)
     with pytest.raises(SparseError):
         gpu.coo_csr(A)
+
+
+def _long(kind):
+    rng = np.random.default_rng(2)
+    if kind == "radix":     # one row beyond a bucket, found by the count
+        return _lens("radix")
+    if kind == "hub":       # found by the sample before it
+        return np.concatenate([rng.integers(0, 12, 150_000), [120_000], rng.integers(0, 12, 50_000)])
+    if kind == "hubs":      # missed or met by the sample, as it falls
+        return np.concatenate([rng.integers(0, 12, 100_000), np.full(5, 13_000),
+                               rng.integers(0, 12, 100_000)])
+    # a bucket that has to be cut down to rows of their own
+    return np.concatenate([rng.integers(0, 3, 40_000), np.full(9, 8192), rng.integers(0, 3, 9_000)])
+
+
+def _sorted(row, col, val, N):
+    """The stable sort by (row, col) that coo_csr is (the oracle's bubble sort
+    takes minutes on rows of this length)."""
+    p = np.lexsort((col, row))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(row, minlength=N))]).astype(np.int32)
+    return rp, col[p], val[p]
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("kind", ["radix", "hub", "hubs", "own"])
+def test_rows_beyond_buckets(gpu, dt, kind):
+    """coo_csr with such rows, and the transpose with such columns."""
+    lens = _long(kind)
+    N = lens.size
+    row, col, val = _coo(lens, N, 7, 0.2)
+    val = val.astype(dt)
+    A = gpu.coo_csr(gpu.coo_from_host(row, col, val, N))
+    for got, w in zip((A.row_array(), A.col_array(), A.val_array()), _sorted(row, col, val, N)):
+        assert np.array_equal(_ub(got), _ub(w)), kind
+    rp, c, v = _sorted(col, row, val, N)
+    B = gpu.transpose(gpu.csr_from_host(rp, c, v))
+    at = np.repeat(np.arange(N, dtype=np.int32), np.diff(rp))
+    for got, w in zip((B.row_array(), B.col_array(), B.val_array()), _sorted(c, at, v, N)):
+        assert np.array_equal(_ub(got), _ub(w)), kind
+
+
+@pytest.mark.parametrize("bad", [-1, 200_001, 2**31 - 1])
+def test_index_out_of_range_beside_a_hub(gpu, bad):
+    """The sample ends the count; the indices are checked all the same."""
+    lens = _long("hub")
+    N = lens.size
+    row, col, val = _coo(lens, N, 9)
+    A = gpu.coo_from_host(row, col, val, N)
+    col[-1000] = bad
+    A.col_index.upload(col)
+    with pytest.raises(SparseError):
+        gpu.coo_csr(A)
