@@ -132,6 +132,19 @@ def test_rows_beyond_buckets(gpu, dt, kind):
         assert np.array_equal(_ub(got), _ub(w)), kind
 
 
+@pytest.mark.parametrize("N,per_row", [(3, 500), (1000, 65), (9471, 9), (30_011, 20), (320_001, 3)])
+def test_transpose_rows_per_warp(gpu, N, per_row):
+    """One row to a warp up to 32, the last warp with fewer, empty rows between."""
+    rng = np.random.default_rng(N)
+    lens = np.where(rng.random(N) < 0.1, 0, rng.integers(0, 2 * per_row, N))
+    row = np.repeat(np.arange(N, dtype=np.int32), lens)
+    rp, c, v = _sorted(row, rng.integers(0, N, row.size).astype(np.int32),
+                       rng.uniform(-1, 1, row.size), N)
+    B = gpu.transpose(gpu.csr_from_host(rp, c, v))
+    for got, w in zip((B.row_array(), B.col_array(), B.val_array()), _sorted(c, row, v, N)):
+        assert np.array_equal(_ub(got), _ub(w))
+
+
 @pytest.mark.parametrize("bad", [-1, 200_001, 2**31 - 1])
 def test_index_out_of_range_beside_a_hub(gpu, bad):
     """The sample ends the count; the indices are checked all the same."""
