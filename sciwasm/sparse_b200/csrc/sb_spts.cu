@@ -746,7 +746,7 @@ __global__ void spts_hybrid_rows(const int* __restrict__ rrow, const int* __rest
                                  const T* __restrict__ b, T* yw, T* __restrict__ y,
                                  int* __restrict__ ticket, long long limit, int* status) {
   while (true) {
-    const int base = next_rows(ticket);
+    const int base = next_rows(ticket) + 1;  // (-1 at first, as all pending words)
     if (base >= N) return;
     const int i = base + (threadIdx.x & 31);
     if (i < N) {
@@ -775,7 +775,7 @@ __global__ void spts_syncfree_plan_rows(const int* __restrict__ row_ptr,
                                         int N, const T* __restrict__ b, T* yw, T* __restrict__ y,
                                         int* __restrict__ ticket, long long limit, int* status) {
   while (true) {
-    const int base = next_rows(ticket);
+    const int base = next_rows(ticket) + 1;  // (-1 at first, as all pending words)
     if (base >= N) return;
     const int i = base + (threadIdx.x & 31);
     if (i < N) {
@@ -1285,8 +1285,9 @@ static int solve_impl(const sb_spts_plan* p, int algo, const T* b, T* y, long lo
     SB_CHECK_LAUNCH("spts_level_block");
     return SB_OK;
   }
-  SB_CHECK_CUDA(cudaMemsetAsync(yw, 0xff, sizeof(T) * N, st));
-  SB_CHECK_CUDA(cudaMemsetAsync(p->ticket, 0, sizeof(int), st));
+  // pending values, and the ticket behind them, in one call (with two, a level
+  // solve of few wide levels took 4 us longer than by its former grid barriers)
+  SB_CHECK_CUDA(cudaMemsetAsync(yw, 0xff, (size_t)((char*)(p->ticket + 1) - (char*)yw), st));
   if (algo == SB_SPTS_SYNCFREE) {
     auto k = spts_syncfree_plan_rows<T, A>;
     k<<<polling_grid((const void*)k, algo, N, p->nlevels), kT, 0, st>>>(
