@@ -26,8 +26,8 @@
 //                    src/parallel/src/sparse_opt_32.wat:12846-13445
 // SB_SPTS_LEVEL and SB_SPTS_HYBRID have the same arithmetic, so the kernel is
 // chosen by the factor's shape (solve_impl): one block with its values in
-// shared memory (sb_spts_window.cuh), one block with a barrier per level, or
-// ready flags over the whole GPU.
+// shared memory (sb_spts_window.cuh), a launch per level where there are few,
+// one block with a barrier per level, or ready flags over the whole GPU.
 #include <algorithm>
 #include <climits>
 #include <cstring>
@@ -602,6 +602,33 @@ __global__ void reorder_rows(const int* __restrict__ row_ptr, const int* __restr
 }
 
 // ------------------------------------------------------------ solves
+
+// One level of few: a launch each, a thread per row, with nothing to wait for
+// and no pending values to fill in.  Up to kFewLevels the launches cost less than
+// the ready flags, or a grid barrier per level (the whole call of 1M FP64 rows on
+// B200, flags / grid barriers / so: 1 level 55 / 43 / 32 us, 3 levels 65 / 56 / 42).
+constexpr int kFewLevels = 4;
+
+template <typename T, typename A>
+__global__ void spts_level_rows(const int* __restrict__ rrow, const int* __restrict__ rcol,
+                                const T* __restrict__ rval, const int* __restrict__ level_ptr,
+                                int l, const int* __restrict__ perm, const T* __restrict__ b,
+                                T* yw, T* __restrict__ y) {
+  const int i = level_ptr[l] + (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (i >= level_ptr[l + 1]) return;
+  const int s = rrow[i], end = rrow[i + 1] - 1, pi = perm[i];
+  const A bi = (A)b[pi];
+  T yi;
+  if (end > s) {
+    A t = 0;
+    for (int j = s; j < end; ++j) t = add_rn(t, mul_rn((A)rval[j], (A)yw[rcol[j]]));
+    yi = (T)div_rn(sub_rn(bi, t), (A)rval[end]);
+  } else {
+    yi = (T)div_rn(bi, (A)rval[end]);
+  }
+  yw[i] = yi;
+  y[pi] = yi;
+}
 
 // A thread's first row of a level, read ahead of the barrier that opens the
 // level: its structure, b, diagonal and up to kG off-diagonal columns and
@@ -1275,6 +1302,14 @@ static int solve_impl(const sb_spts_plan* p, int algo, const T* b, T* y, long lo
   if (algo != SB_SPTS_SYNCFREE && p->window.use)
     return solve_window<T, A>(p, b, y, status, st);
   T* yw = (T*)p->ywork;
+  if (algo != SB_SPTS_SYNCFREE && p->nlevels <= kFewLevels) {
+    for (int l = 0; l < p->nlevels; ++l) {
+      spts_level_rows<T, A><<<grid1(p->window.rows), kT, 0, st>>>(
+          p->rrow, p->rcol, (const T*)p->rval, p->level_ptr, l, p->perm, b, yw, y);
+      SB_CHECK_LAUNCH("spts_level_rows");
+    }
+    return SB_OK;
+  }
   if (algo == SB_SPTS_LEVEL && p->window.rows <= kLevelBlock) {
     // the two-round prefetch except for FP32 sums, where the one-round form
     // measured faster (1M-row random factor, 3470 levels: 6.54 against 7.27
@@ -1285,8 +1320,7 @@ static int solve_impl(const sb_spts_plan* p, int algo, const T* b, T* y, long lo
     SB_CHECK_LAUNCH("spts_level_block");
     return SB_OK;
   }
-  // pending values, and the ticket behind them, in one call (with two, a level
-  // solve of few wide levels took 4 us longer than by its former grid barriers)
+  // pending values, and the ticket behind them, in one call
   SB_CHECK_CUDA(cudaMemsetAsync(yw, 0xff, (size_t)((char*)(p->ticket + 1) - (char*)yw), st));
   if (algo == SB_SPTS_SYNCFREE) {
     auto k = spts_syncfree_plan_rows<T, A>;

@@ -166,3 +166,44 @@ def test_dependency_wait_times_out_and_device_stays_usable(gpu, oracle):
     gpu.spts_csr_sync_free(G, gpu.vec_from_host(b), yv)
     assert np.array_equal(_ub(yv.array()), _ub(oracle.spts_syncfree(good_rp, good_col,
                                                                      good_val, b)))
+
+
+@pytest.mark.parametrize("dt,policy", [(np.float32, "native"), (np.float64, "native"),
+                                       (np.float32, "f64")])
+@pytest.mark.parametrize("nlevels", [1, 2, 4, 5])
+def test_few_wide_levels(gpu, oracle, dt, policy, nlevels):
+    """Levels too wide for one block and few enough for a launch each (and one
+    more): bit for bit, in place too."""
+    w = 20_011
+    N = nlevels * w
+    i = np.arange(N)
+    rng = np.random.default_rng(nlevels)
+    deps = [np.where(i >= w, i - w, -1), np.where(i >= w, (i // w - 1) * w + rng.integers(0, w, N), -1)]
+    row = np.concatenate([i, i, i])
+    col = np.concatenate([*deps, i])
+    keep = np.unique(row[col >= 0].astype(np.int64) * N + col[col >= 0])
+    row, col = keep // N, (keep % N).astype(np.int32)
+    rp = np.concatenate([[0], np.cumsum(np.bincount(row, minlength=N))]).astype(np.int32)
+    val = np.where(row == col, 3.0, rng.uniform(-0.3, 0.3, col.size)).astype(dt)
+    b = synth.uniform_vec(N, 4, dtype=dt)
+    if policy == "native":
+        want = oracle.spts_csr(rp, col, val, b)
+    else:
+        want = np.empty(N, np.float32)  # level by level, entries in order, sums in FP64
+        for l in range(nlevels):
+            r = np.arange(l * w, (l + 1) * w)
+            t = np.zeros(w)
+            for k in range(int((rp[r + 1] - rp[r]).max()) - 1):
+                on = rp[r] + k < rp[r + 1] - 1
+                j = rp[r[on]] + k
+                t[on] = t[on] + val[j].astype(np.float64) * want[col[j]].astype(np.float64)
+            want[r] = ((b[r].astype(np.float64) - t) / val[rp[r + 1] - 1]).astype(np.float32)
+    A = gpu.csr_from_host(rp, col, val)
+    for algo in ("level", "hybrid"):
+        bv, yv = gpu.vec_from_host(b), gpu.create_vec(N, 0, dt)
+        for _ in range(2):
+            gpu.spts(A, bv, yv, algo=algo, policy=policy)
+            assert np.array_equal(_ub(yv.array()), _ub(want)), algo
+        gpu.spts(A, bv, bv, algo=algo, policy=policy)
+        assert np.array_equal(_ub(bv.array()), _ub(want)), algo
+    assert A._plan.nlevels == nlevels
