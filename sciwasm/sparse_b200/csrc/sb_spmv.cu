@@ -301,15 +301,16 @@ __device__ __forceinline__ float ld_val(const __nv_bfloat16* p) {
 // index, value and x wherever the compiler sees fit, which varies from one
 // instance of the row kernel to the next.  The kernel takes ld_if for the
 // whole-warp tail and for short rows of 4 lanes and more, but conditions where
-// those measured faster: V <= 2 (5-point Laplacian of 4M rows bf16, V = 1, 39 us
-// and 50; its tail too, FP64 58 and 61), FP64 with V >= 16 (4M rows of
-// Poisson(40) entries, random columns, 744 and 783), and stores to several
-// arrays, whose 32 registers would spill.  Measured on B200 (us, conditions
+// those measured faster: short rows with V <= 2 (5-point Laplacian of 4M rows
+// bf16, V = 1, 39 us and 50) and the tail beside V = 1 (FP64 58 and 61); FP64 short
+// rows with V >= 16 (4M rows of Poisson(40) entries, random columns, 744 and 783)
+// and, where sums go to several arrays within 32 registers, their tail (41
+// diagonals of 4M rows 503 and 585).  Measured on B200 (us, conditions
 // everywhere -> now): rows of 5 + Zipf(2) entries, 1M of them, f32 92 -> 74, FP64
-// 101 -> 83; of 15 + Zipf(2), 4M, 367 -> 359 and 423 -> 404; 41 diagonals of 1M rows
-// f32 112 -> 72; 27-point stencil of 4M rows f32 184 -> 171, FP64 273 -> 261; 15
-// diagonals FP64 206 -> 183.  What lost: 7-point stencil FP64 77 -> 80, 9-point
-// 89 -> 92.
+// 101 -> 83; of 15 + Zipf(2), 4M, 367 -> 359 and 423 -> 404; 41 diagonals of 1M
+// rows f32 112 -> 72; 27-point stencil of 4M rows f32 184 -> 171, FP64 273 -> 261;
+// 15 diagonals FP64 206 -> 183.  What lost: 7-point stencil FP64 77 -> 80, 9-point
+// 89 -> 92; to several arrays, Poisson(20) FP64 419 -> 435.
 __device__ __forceinline__ int ld_if(const int* p, bool on) {
   int v;
   asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %2, 0;\nmov.b32 %0, 0;\n"
@@ -409,7 +410,7 @@ __device__ __forceinline__ void csr_short_rows(const int* __restrict__ col,
                                                int r0, int s_l, int e_l, T y_l) {
   constexpr int RPB = kWarp / V;     // rows per batch
   constexpr int PASS = V * UNROLL;   // entries of one unrolled pass
-  constexpr bool PRED = !Out::kAll && (sizeof(T) == 4 ? V > 2 : V == 4 || V == 8);  // see ld_if
+  constexpr bool PRED = sizeof(T) == 4 ? V > 2 : V == 4 || V == 8;  // see ld_if
   const int lane = threadIdx.x & (kWarp - 1);
   const int g = lane / V;
   const int q = lane - g * V;
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(256, Out::template min_blocks<T>())
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int k = k0 + lane + u * kWarp;
-          if constexpr (V == 1 || Out::kAll) {
+          if constexpr (V == 1 || (Out::kAll && sizeof(T) == 8 && V >= 16)) {
             cc[u] = k < e ? ld_reuse(col + k) : 0;
             vv[u] = k < e ? (T)ld_val_reuse(val + k) : (T)0;
           } else {
