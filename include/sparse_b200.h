@@ -372,7 +372,8 @@ int sb_dia_admitted(int64_t ndiags, int32_t stride, int64_t nnz);
 /* Replaces the fill of csr_dia (src/sequential/src/sparse32.js:1515-1574):
  * offset[nd] ascending, data[nd*stride] diagonal-major (zero where no entry),
  * a later duplicate (i, c) in row order overwriting an earlier one.  Returns
- * SB_EREFUSED where the reference returns undefined. */
+ * SB_EREFUSED where the reference returns undefined, and SB_EINVAL for an nd
+ * that is not the matrix's; offset and data may have been written by then. */
 int sb_csr_dia(int dtype, const int32_t* row_ptr, const int32_t* col, const void* val, int32_t N,
                int64_t nnz, int32_t nd, int32_t stride, int32_t* offset, void* data,
                void* stream);
