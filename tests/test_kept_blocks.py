@@ -75,14 +75,14 @@ int main() {
   bool twice;
   void* p[17];
   for (void*& q : p) q = get(k, MIB);
-  for (int i = 0; i < 15; ++i) put(k, p[i]);
+  constexpr int few = (int)Kept::kEnoughSame - 1;
+  for (int i = 0; i < few; ++i) put(k, p[i]);
   int m = Fake::mallocs, f = Fake::frees;
-  void* fresh = get(k, MIB);  // 15 of the size: a new block, no wait
+  void* fresh = get(k, MIB);  // too few of the size: a new block, no wait
   CHECK(Fake::mallocs == m + 1 && Fake::frees == f);
-  put(k, p[15]);
-  put(k, p[16]);
+  for (int i = few; i < 17; ++i) put(k, p[i]);
   CHECK(k.free(p[16], &twice) == 0 && twice);
-  // 17: the first freed one, after a free by the driver
+  // enough: the first freed one, after a free by the driver
   std::promise<void*> got;
   std::thread t([&] { Fake::held_up = true; got.set_value(get(k, MIB)); });
   while (!Fake::waiting) std::this_thread::yield();
