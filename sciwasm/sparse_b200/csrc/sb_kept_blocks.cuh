@@ -17,12 +17,13 @@
 //     then does an allocation wait.  (A plan of 30,000 rows takes 0.61 ms with a
 //     new block and 0.26 with a kept one, from the fifth on; with 16 blocks of a
 //     size, as a dearer wait had wanted it, from the 17th, and with four times
-//     the memory.  Passes of conversions take as long with either.)  The wait is a cudaMalloc and cudaFree of 16
-//     bytes beside a small block held for good: the driver carves small blocks
-//     out of 2 MiB chunks, and the pair takes 4 us on an idle B200 where a chunk
-//     is open, 1300 us where it maps and unmaps one.  (Blocks under 2 MiB
-//     themselves cost the driver about as little, so with the dearer wait
-//     coo_csr of 88k entries took 200 us a call against 190 without kept blocks.)
+//     the memory.  Passes of conversions take as long with either.)
+//     The wait is a cudaMalloc and cudaFree of 16 bytes beside a small block held
+//     for good: the driver carves small blocks out of 2 MiB chunks, and the pair
+//     takes 4 us on an idle B200 where a chunk is open, 1300 us where it maps and
+//     unmaps one.  (Blocks under 2 MiB themselves cost the driver about as little,
+//     so with the dearer wait coo_csr of 88k entries took 200 us a call against
+//     190 without kept blocks.)
 //   * Kept blocks are given back to the driver when an allocation of this
 //     library fails, before it is tried once more; sb_mem_info counts them as
 //     free.
