@@ -139,6 +139,7 @@ constexpr int kKnownRows = 512;  // at each end
 struct Known {
   int count;  // of the first and last rows; kDiaGather + 1: more
   int stray;  // set: a row has a diagonal outside offset[0 .. count)
+  int check;  // set: a diagonal's byte is read before it is stored (mark_all)
   int offset[kDiaGather];
 };
 
@@ -160,9 +161,17 @@ __device__ __forceinline__ void insert_offset(int d, int* key, int* count) {
   }
 }
 
+// present (zero on entry; may be null): where there are too many for the list, the
+// diagonals of a few rows are marked ahead of all others, so that the warps
+// of mark_all that start together find the bytes of a wide stencil set instead of
+// all storing to the same few sectors; and they tell whether rows share their
+// diagonals at all.
+constexpr int kSeedRows = 8;        // of the middle
+constexpr int kSeedEntries = 1024;  // of a row at most
+
 __global__ void __launch_bounds__(2 * kKnownRows)
     known_diagonals(const int* __restrict__ row_ptr, const int* __restrict__ col, int N,
-                    Known* __restrict__ known) {
+                    Known* __restrict__ known, unsigned char* __restrict__ present) {
   __shared__ int key[kSlots];
   __shared__ int count;
   const int t = threadIdx.x;
@@ -202,6 +211,33 @@ __global__ void __launch_bounds__(2 * kKnownRows)
     for (int k = 0; k < kSlots; ++k) rank += key[k] < key[t];
     known->offset[rank] = key[t];
   }
+  if (n > kDiaGather && present) {
+    // one warp to a row: four from the middle, the first and the last four (where
+    // one-sided diagonals begin), then the next four of the middle, held against
+    // what the others marked
+    __shared__ int seen, all;
+    if (t == 0) seen = all = 0;
+    __syncthreads();
+    const int w = t >> 5;
+    const int r = w < kSeedRows ? N / 2 + w : w < 12 ? w - kSeedRows : N - 1 - (w - 12);
+    const bool mine = w < 16 && r >= 0 && r < N;
+    const int s0 = mine ? row_ptr[r] : 0, len = mine ? min(row_ptr[r + 1] - s0, kSeedEntries) : 0;
+    for (int half = 0; half < 2; ++half) {
+      if ((w >= 4 && w < kSeedRows) == (half == 1))
+        for (int j = t & 31; j < len; j += 32) {
+          const int c = col[s0 + j];
+          if ((unsigned)c >= (unsigned)N) continue;
+          unsigned char* f = present + ((long long)N + c - r - 1);
+          if (half) {
+            atomicAdd(&all, 1);
+            if (*(volatile unsigned char*)f) atomicAdd(&seen, 1);
+          }
+          *f = 1;
+        }
+      __syncthreads();
+    }
+    if (t == 0) known->check = 2 * seen > all;
+  }
 }
 
 // The first of n ascending offsets that is not below d.
@@ -229,17 +265,21 @@ __device__ __forceinline__ bool run_of_offsets(const int* __restrict__ col, int 
 // Every diagonal of the rows into present: a warp takes `rows` (at most 32)
 // rows at a time and its lanes their entries in storage order, so that loads
 // coalesce and long rows are shared out; an entry's row is found among the
-// row pointers.  Where 32 entries in a row lie on near diagonals (a band, a
-// dense block) a byte is stored only while it reads 0 (a stale 0 costs one
-// more idempotent store), as the same few sectors would otherwise be stored
-// over and over; elsewhere the check would be a round trip for nothing.
-// num_diags on B200, host time: 200k rows of 81 diagonals, checking 0.14 ms,
-// storing plainly 0.30; 2M-row power law of 38M entries 0.56 and 0.44; with
-// 4-byte flags and a thread per row 0.25 and 0.52.
+// row pointers.  A byte is stored only while it reads 0 (a stale 0 costs one
+// more idempotent store) where rows share their diagonals (known->check) or 32
+// entries in a row lie on near ones, as the same few sectors would otherwise be
+// stored over and over; elsewhere the check would be a round trip for nothing.
+// num_diags on B200, the whole call in us (4-byte flags and a thread per row /
+// bytes checked on near diagonals alone / now): 30,000 rows of 80 diagonals 97 /
+// 77-130 / 58, 300,000 rows 307 / 134 / 121; 100 diagonals 97 apart, 300,000 rows
+// 187 / 8960 / 143; 125-point stencil of 1.5M rows 757 / 5025 / 563; power law of 2M
+// rows 529 / 430 / 430.  Random columns lose what the bytes save on structure: 60
+// entries a row, 300,000 rows 222 / 290 / 290 (checked 315), 10,000 rows 88 / 178 /
+// 178 (checked 253).
 constexpr int kNarrow = 4096;
 
 __device__ void mark_all(const int* __restrict__ row_ptr, const int* __restrict__ col, int N,
-                         int rows, int (*ptr)[33], unsigned char* present) {
+                         int rows, bool always, int (*ptr)[33], unsigned char* present) {
   const int lane = threadIdx.x & 31;
   int* p = ptr[threadIdx.x >> 5];
   const int warps = gridDim.x * (kThreads / 32);
@@ -278,7 +318,7 @@ __device__ void mark_all(const int* __restrict__ row_ptr, const int* __restrict_
       }
       const unsigned lo = __reduce_min_sync(0xffffffffu, at[0] >= 0 ? (unsigned)at[0] : ~0u);
       const unsigned hi = __reduce_max_sync(0xffffffffu, at[0] >= 0 ? (unsigned)at[0] : 0u);
-      const bool check = hi - lo < (unsigned)kNarrow;
+      const bool check = always || hi - lo < (unsigned)kNarrow;
 #pragma unroll
       for (int u = 0; u < kAhead; ++u)
         have[u] = at[u] >= 0 ? (check ? present[at[u]] : (unsigned char)0) : (unsigned char)1;
@@ -298,7 +338,7 @@ __global__ void __launch_bounds__(kThreads)
   __shared__ int ptr[kThreads / 32][33];
   const int n = known->count;
   if (n > kDiaGather) {
-    mark_all(row_ptr, col, N, rows, ptr, present);
+    mark_all(row_ptr, col, N, rows, known->check, ptr, present);
     return;
   }
   if (threadIdx.x < n) {
@@ -584,7 +624,7 @@ static int find_diagonals(const int* row_ptr, const int* col, int N, const Diags
                           int* nd, cudaStream_t st) {
   unsigned char* present = reinterpret_cast<unsigned char*>(d.present);
   SB_CHECK_CUDA(cudaMemsetAsync(present, 0, sizeof(uint4) * (size_t)d.words, st));
-  known_diagonals<<<1, 2 * kKnownRows, 0, st>>>(row_ptr, col, N, d.known);
+  known_diagonals<<<1, 2 * kKnownRows, 0, st>>>(row_ptr, col, N, d.known, present);
   const unsigned grid = (unsigned)sm_count() * 8;
   // rows a warp of mark_all takes: as many as leave every warp some, 1 to 32
   int rows = 32;
@@ -625,7 +665,7 @@ static int csr_dia_known(const int* row_ptr, const int* col, const T* val, int N
   int r = scratch_alloc((void**)&known, sizeof(Known), st);
   if (r) return r;
   int head[2] = {0, 0};
-  known_diagonals<<<1, 2 * kKnownRows, 0, st>>>(row_ptr, col, N, known);
+  known_diagonals<<<1, 2 * kKnownRows, 0, st>>>(row_ptr, col, N, known, nullptr);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(head, known, sizeof(head), cudaMemcpyDeviceToHost, st);

@@ -109,3 +109,35 @@ def test_row_pointers_that_do_not_ascend(gpu, oracle, width):
     ascending = rp.copy()        # (the host check of an upload refuses the others)
     rp[200:3000:301] -= 2 * width + 1  # rows before these are empty, these overlap older entries
     assert _check(gpu, oracle, rp, col, val, ascending)
+
+
+@pytest.mark.parametrize("N", [70, 137, 4000, 30_000])
+@pytest.mark.parametrize("kind", ["far", "alternating", "random", "long_middle", "empty_middle"])
+def test_many_diagonals_and_middle_rows(gpu, oracle, N, kind):
+    """More diagonals than the list holds, with the middle rows (which are marked
+    first and say whether rows share their diagonals) like the others, alternating,
+    unlike any other, longer than is looked at, or empty."""
+    rng = np.random.default_rng(N)
+    step = max(1, N // 80)
+    offsets = np.arange(0, min(100, N) * step, step)[:100] if kind != "random" else np.arange(0)
+    if kind == "random":
+        rows = np.repeat(np.arange(N), 8)
+        col = rng.integers(0, N, rows.size)
+    else:
+        rows = np.repeat(np.arange(N), offsets.size)
+        col = (rows + np.tile(offsets, N)) % N
+        if kind == "alternating":  # three kinds of rows in turn
+            keep = np.tile(np.arange(offsets.size) % 3, N) == rows % 3
+            rows, col = rows[keep], col[keep]
+    mid = (rows >= N // 2) & (rows < N // 2 + 8)
+    if kind in ("long_middle", "empty_middle"):
+        rows, col = rows[~mid], col[~mid]
+    if kind == "long_middle":
+        extra = np.repeat(np.arange(N // 2, min(N, N // 2 + 8)), min(N, 2000))
+        rows, col = np.concatenate([rows, extra]), np.concatenate([col, rng.integers(0, N, extra.size)])
+    p = np.lexsort((col, rows))
+    rows, col = rows[p], col[p]
+    rp = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=N))]).astype(np.int32)
+    A = gpu.csr_from_host(rp, col.astype(np.int32), rng.standard_normal(col.size).astype(np.float32))
+    for _ in range(3):
+        assert gpu.num_diags(A) == [np.unique(col - rows).size, N]
